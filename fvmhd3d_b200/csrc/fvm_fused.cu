@@ -76,32 +76,6 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned &gen, int *
 
 __device__ __forceinline__ int vload(const int *p) { return *reinterpret_cast<const volatile int *>(p); }
 
-// The ascending list of the step's active non-boundary sites (site flag set
-// by the mark stage), compacted from the ascending involved-cell list by one
-// block: the order the sequential adjust_timesteps sweep visits them in.
-__device__ void compact_sites(const int *clist, int ninv, const unsigned char *site, int *alist) {
-  __shared__ int wsum[32];
-  __shared__ int base;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if (threadIdx.x == 0) base = 0;
-  __syncthreads();
-  for (int c0 = 0; c0 < ninv; c0 += blockDim.x) {
-    const int t = c0 + threadIdx.x;
-    const int i = t < ninv ? clist[t] : -1;
-    const bool f = i >= 0 && site[i] != 0;
-    const unsigned b = __ballot_sync(0xffffffffu, f);
-    if (lane == 0) wsum[w] = __popc(b);
-    __syncthreads();
-    int o = base;
-    for (int k = 0; k < w; k++) o += wsum[k];
-    if (f) alist[o + __popc(b & ((1u << lane) - 1u))] = i;
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int k = 0; k < nw; k++) base += wsum[k];
-    __syncthreads();
-  }
-}
-
 // One partial step, limiter to reconstruction (the stage kernels' order in
 // enq_limiter .. enq_recon), exact flux.  The step's active-face and
 // involved-cell lists are built before the launch; never every cell is
@@ -182,37 +156,29 @@ __global__ void __launch_bounds__(128, FVM_FLUX_MINB(R)) k_rung_step(FusedStep a
   FVM_GRID_SYNC();
   adjust_mark_group<kCellGroup>(d.off, d.lfj, d.act, d.bnd, d.dtl, d.hash, &S->iscal[4], d.act0, d.awork, d.clist,
                                 S->ninv, gl, gmask, gt / kCellGroup, gn / kCellGroup);
-  {  // active non-boundary sites (the count the separate-kernel step takes from its compaction)
-    const int ninv = S->ninv;
-    int cnt = 0;
-    for (int t = gt; t < ninv; t += gn) cnt += d.act0[d.clist[t]] != 0;  // sites this thread marked
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(&S->iscal[5], cnt);
-  }
   FVM_GRID_SYNC();
   adjust_init_dev<kCellGroup>(n, d.off, d.lfj, d.act, &S->iscal[4], d.dtl, d.dt0, d.rdv, d.wrv, d.aflag, d.clist,
                               &S->ninv, gt, gn);
   FVM_GRID_SYNC();
   bool settled = false;
   for (int k = 0; k < ADJ_ITERS; k++) {
-    adjust_replay_dev(n, k, d.off, d.lfj, d.lsort, d.lpart, d.act, d.dt0, d.rdv, d.wrv, d.dtl, d.aflag, d.awork, 0, gt,
+    adjust_replay_dev<ADJ_LANES>(n, k, d.off, d.lfj, d.lsort, d.lpart, d.act, d.dt0, d.rdv, d.wrv, d.dtl, d.aflag, d.awork, 0, gt,
                       gn, d.clist, S->ninv);
     FVM_GRID_SYNC();
     // stop once replay k changed nothing (settled) or every replay has run
     settled = vload(&d.aflag[k % 3]) == 0;
     if (settled || k + 1 >= ADJ_ITERS) break;
   }
-  // adjust_restore_dev's decision, taken by every block from the same flags:
-  // the sequential sweep runs from the initial timesteps when the replays did
-  // not settle; otherwise the replays' timesteps stand and no barrier is
-  // needed before the rungs
+  // k_adjust_seq's decision, taken by every block from the same flags: the
+  // sequential sweep runs from the initial timesteps when the replays did not
+  // settle; otherwise the replays' timesteps stand and no barrier is needed
+  // before the rungs
   {
     const bool fallback = !settled && vload(&d.aflag[(ADJ_ITERS - 1) % 3]) != 0;
     if (gt == 0) {
       if (settled) d.aflag[5] = 1;
       S->iscal[6] = vload(&d.aflag[3]);
       S->iscal[7] = fallback ? 1 : 0;
-      if (fallback) d.aflag[4] = 1;
     }
     if (fallback) {
       const int ninv = S->ninv;
@@ -222,9 +188,8 @@ __global__ void __launch_bounds__(128, FVM_FLUX_MINB(R)) k_rung_step(FusedStep a
       }
       FVM_GRID_SYNC();
       if (blockIdx.x == 0) {  // not settled: the sequential sweep
-        compact_sites(d.clist, S->ninv, d.act0, d.alist);
-        __syncthreads();
-        if (threadIdx.x == 0) adjust_seq_dev(d.off, d.lnk, d.s12, d.alist, &S->iscal[5], &d.aflag[4], d.dtl);
+        const int nsites = compact_sites(d.clist, S->ninv, n, d.act0, d.alist);
+        if (threadIdx.x == 0) adjust_seq_dev(d.off, d.lnk, d.s12, d.alist, nsites, d.dtl);
       }
       FVM_GRID_SYNC();
     }
