@@ -37,6 +37,8 @@ struct Sched {
   int inc[2];  // incremental list building: [0] links of the active cells, [1] 1 when
                // this step's lists were built that way
   unsigned long long inc_steps;  // steps whose lists were built incrementally
+  int ff_all;                 // the face flags are those of every cell active (no partial step since)
+  int ff_count;               // active faces of those flags
 };
 
 struct Dev {
@@ -219,8 +221,15 @@ enum : unsigned char { FF_ACTIVE = 1, FF_BND1 = 2, FF_BND2 = 4 };
 __global__ void k_faceflags(int nf, const int2 *FVM_RESTRICT s12, unsigned char *FVM_RESTRICT act,
                             const int *FVM_RESTRICT bnd, unsigned char *FVM_RESTRICT fflag,
                             int *FVM_RESTRICT nface_active, unsigned char *FVM_RESTRICT fcode,
-                            unsigned char *FVM_RESTRICT fcode2, int *FVM_RESTRICT bcount) {
+                            unsigned char *FVM_RESTRICT fcode2, int *FVM_RESTRICT bcount, Sched *FVM_RESTRICT S,
+                            int n) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  // a global step after one with every cell active: the flags stand (they
+  // follow from the active cells and the boundary codes alone)
+  if (!bcount && S->ff_all && S->iscal[1] == n) {
+    if (f == 0) *nface_active = S->ff_count;
+    return;
+  }
   bool a = false;
   if (f < nf) {
     const int2 e = s12[f];
@@ -918,32 +927,6 @@ __device__ __forceinline__ void limiter_st_block(int cb, int n, bool reuse, doub
   }
 }
 
-// One block per CST cells; with only_all set (partial-step mode) the kernel
-// does nothing unless every cell is active this step, the case k_limiter's
-// list then skips.
-template <typename R, int KH, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_limiter_st(int n, Params P, const Sched *FVM_RESTRICT S,
-    const int *FVM_RESTRICT off, const int *FVM_RESTRICT lnk, const int2 *FVM_RESTRICT lfj, const int2 *FVM_RESTRICT s12,
-    const double4 *FVM_RESTRICT geo, const double4 *FVM_RESTRICT dr1, const unsigned char *FVM_RESTRICT fflag,
-    const unsigned char *FVM_RESTRICT act, const double *FVM_RESTRICT tlast,
-    const R *FVM_RESTRICT Wrec, R *FVM_RESTRICT tau, R *FVM_RESTRICT fst, const int *FVM_RESTRICT perm,
-    const R *FVM_RESTRICT mnmx, const unsigned char *FVM_RESTRICT mz, int only_all, const R *FVM_RESTRICT lld) {
-  constexpr int CST = limiter_cst<KH>();
-  extern __shared__ __align__(16) unsigned char lsm[];
-  __shared__ int soff[CST + 1];
-  if (only_all && S->iscal[1] != n) return;
-  const double t_global = S->t_global;
-  const bool reuse = FVM_REUSE_MINMAX && S->mnmx_ok && S->iscal[1] == n;
-  // one cell block per block, or (a grid smaller than the cell blocks, as
-  // partial steps launch it, where it usually has nothing to do) a loop over
-  // them; a block's threads meet at the block's barriers in every pass
-  const int ncb = (n + CST - 1) / CST;
-  for (int cb = blockIdx.x; cb < ncb; cb += gridDim.x) {
-    if (cb != (int)blockIdx.x) __syncthreads();  // the previous pass is done with the staging
-    limiter_st_block<R, KH>(cb, n, reuse, t_global, soff, lsm, off, lnk, lfj, s12, geo, dr1, fflag, act, tlast,
-                            Wrec, tau, fst, perm, mnmx, mz, lld);
-  }
-}
 template <typename R, int KH, int MINB>
 __device__ __forceinline__ void limiter_dev(int n, Params P, const Sched *FVM_RESTRICT S,
     const int *FVM_RESTRICT off, const int *FVM_RESTRICT lnk, const int2 *FVM_RESTRICT lfj, const int2 *FVM_RESTRICT s12,
@@ -951,8 +934,7 @@ __device__ __forceinline__ void limiter_dev(int n, Params P, const Sched *FVM_RE
     const unsigned char *FVM_RESTRICT act, const double *FVM_RESTRICT tlast,
     const R *FVM_RESTRICT Wrec, R *FVM_RESTRICT tau, R *FVM_RESTRICT fst, const int *FVM_RESTRICT perm,
     const R *FVM_RESTRICT mnmx, const unsigned char *FVM_RESTRICT mz, const int *FVM_RESTRICT clist,
-    int skip_if_all, const R *FVM_RESTRICT lld, int gt0_, int gnt_) {
-  if (skip_if_all && S->iscal[1] == n) return;  // the staged limiter has this step
+    const R *FVM_RESTRICT lld, int gt0_, int gnt_) {
   const double t_global = S->t_global;
   // every cell steps and every cell was reconstructed by the last step: the
   // neighbour min/max of pass 1 are the reconstruction's (same states, same
@@ -976,10 +958,40 @@ __global__ void __launch_bounds__(128, MINB) k_limiter(int n, Params P, const Sc
     const unsigned char *FVM_RESTRICT act, const double *FVM_RESTRICT tlast,
     const R *FVM_RESTRICT Wrec, R *FVM_RESTRICT tau, R *FVM_RESTRICT fst, const int *FVM_RESTRICT perm,
     const R *FVM_RESTRICT mnmx, const unsigned char *FVM_RESTRICT mz, const int *FVM_RESTRICT clist,
-    int skip_if_all, const R *FVM_RESTRICT lld) {
-  limiter_dev<R, KH, MINB>(n, P, S, off, lnk, lfj, s12, geo, dr1, fflag, act, tlast, Wrec, tau, fst, perm, mnmx, mz, clist, skip_if_all, lld, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    const R *FVM_RESTRICT lld) {
+  limiter_dev<R, KH, MINB>(n, P, S, off, lnk, lfj, s12, geo, dr1, fflag, act, tlast, Wrec, tau, fst, perm, mnmx, mz, clist, lld, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
+// The staged limiter: one block per CST cells.  In partial steps (clist not
+// null) a fixed grid, which stages the cells when every one is active and else
+// walks the involved-cell list, one thread per cell and primitive pair.
+template <typename R, int KH, int MINB>
+__global__ void __launch_bounds__(128, MINB) k_limiter_st(int n, Params P, const Sched *FVM_RESTRICT S,
+    const int *FVM_RESTRICT off, const int *FVM_RESTRICT lnk, const int2 *FVM_RESTRICT lfj, const int2 *FVM_RESTRICT s12,
+    const double4 *FVM_RESTRICT geo, const double4 *FVM_RESTRICT dr1, const unsigned char *FVM_RESTRICT fflag,
+    const unsigned char *FVM_RESTRICT act, const double *FVM_RESTRICT tlast,
+    const R *FVM_RESTRICT Wrec, R *FVM_RESTRICT tau, R *FVM_RESTRICT fst, const int *FVM_RESTRICT perm,
+    const R *FVM_RESTRICT mnmx, const unsigned char *FVM_RESTRICT mz, const int *FVM_RESTRICT clist, const R *FVM_RESTRICT lld) {
+  constexpr int CST = limiter_cst<KH>();
+  extern __shared__ __align__(16) unsigned char lsm[];
+  __shared__ int soff[CST + 1];
+  if (clist && S->iscal[1] != n) {
+    limiter_dev<R, KH, MINB>(n, P, S, off, lnk, lfj, s12, geo, dr1, fflag, act, tlast, Wrec, tau, fst, perm, mnmx, mz,
+                             clist, lld, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    return;
+  }
+  const double t_global = S->t_global;
+  const bool reuse = FVM_REUSE_MINMAX && S->mnmx_ok && S->iscal[1] == n;
+  // one cell block per block, or (a grid smaller than the cell blocks, in
+  // partial steps) a loop over them; a block's threads meet at the block's
+  // barriers in every pass
+  const int ncb = (n + CST - 1) / CST;
+  for (int cb = blockIdx.x; cb < ncb; cb += gridDim.x) {
+    if (cb != (int)blockIdx.x) __syncthreads();  // the previous pass is done with the staging
+    limiter_st_block<R, KH>(cb, n, reuse, t_global, soff, lsm, off, lnk, lfj, s12, geo, dr1, fflag, act, tlast,
+                            Wrec, tau, fst, perm, mnmx, mz, lld);
+  }
+}
 
 // ---- compute_update face pass (MPI/compute_update.cpp:106-269) -----------
 // One thread per face: half-step extrapolated face states, face velocity,
@@ -1372,65 +1384,16 @@ __device__ __forceinline__ void corr_cell_group(int c, int gl, unsigned gmask, d
                         divb);
 }
 
-// One thread per cell; in partial steps a fixed grid strides over the
-// involved-cell list (clist, count ninv) instead of every cell.
-template <typename R>
-__device__ __forceinline__ void corr_cell_dev(int n, Params P, const Sched *FVM_RESTRICT S,
-    const int *FVM_RESTRICT off, const int2 *FVM_RESTRICT lfj, const int2 *FVM_RESTRICT s12,
-    const double *FVM_RESTRICT cvol, const unsigned char *FVM_RESTRICT act, const int *FVM_RESTRICT bnd,
-    const double *FVM_RESTRICT pos, const double *FVM_RESTRICT tlast, double *FVM_RESTRICT volp,
-    const R *FVM_RESTRICT Wrec, const R *FVM_RESTRICT tau,
-    const R *FVM_RESTRICT fcon, const unsigned char *FVM_RESTRICT fcode,
-    double *FVM_RESTRICT U, double *FVM_RESTRICT dU, double *FVM_RESTRICT stepdU,
-    unsigned long long *FVM_RESTRICT counters, const int *FVM_RESTRICT perm, float *FVM_RESTRICT divb,
-    const int *FVM_RESTRICT clist, int gt0_, int gnt_) {
-  const double t_global = S->t_global;
-  const int cnt = clist ? S->ninv : n;
-  const bool lst = clist && cnt != n;  // every cell involved: the list is the identity
-  for (int t = gt0_; t < cnt; t += gnt_)
-    corr_cell_body<R>(lst ? clist[t] : perm[t], t_global, P, off, lfj, cvol, act, bnd, pos, tlast, volp, Wrec, tau,
-                      fcon, fcode, U, dU, stepdU, counters, divb);
-}
-template <typename R>
-__global__ void __launch_bounds__(128) k_corr_cell(int n, Params P, const Sched *FVM_RESTRICT S,
-    const int *FVM_RESTRICT off, const int2 *FVM_RESTRICT lfj, const int2 *FVM_RESTRICT s12,
-    const double *FVM_RESTRICT cvol, const unsigned char *FVM_RESTRICT act, const int *FVM_RESTRICT bnd,
-    const double *FVM_RESTRICT pos, const double *FVM_RESTRICT tlast, double *FVM_RESTRICT volp,
-    const R *FVM_RESTRICT Wrec, const R *FVM_RESTRICT tau,
-    const R *FVM_RESTRICT fcon, const unsigned char *FVM_RESTRICT fcode,
-    double *FVM_RESTRICT U, double *FVM_RESTRICT dU, double *FVM_RESTRICT stepdU,
-    unsigned long long *FVM_RESTRICT counters, const int *FVM_RESTRICT perm, float *FVM_RESTRICT divb,
-    const int *FVM_RESTRICT clist) {
-  corr_cell_dev<R>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, tlast, volp, Wrec, tau, fcon, fcode, U, dU, stepdU, counters, perm, divb, clist, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
-}
-// The same for global steps, with more resident blocks.
-template <typename R>
-__global__ void __launch_bounds__(128, FVM_CORR_CELL_MINB(R)) k_corr_cell_g(int n, Params P, const Sched *FVM_RESTRICT S,
-    const int *FVM_RESTRICT off, const int2 *FVM_RESTRICT lfj, const int2 *FVM_RESTRICT s12,
-    const double *FVM_RESTRICT cvol, const unsigned char *FVM_RESTRICT act, const int *FVM_RESTRICT bnd,
-    const double *FVM_RESTRICT pos, const double *FVM_RESTRICT tlast, double *FVM_RESTRICT volp,
-    const R *FVM_RESTRICT Wrec, const R *FVM_RESTRICT tau,
-    const R *FVM_RESTRICT fcon, const unsigned char *FVM_RESTRICT fcode,
-    double *FVM_RESTRICT U, double *FVM_RESTRICT dU, double *FVM_RESTRICT stepdU,
-    unsigned long long *FVM_RESTRICT counters, const int *FVM_RESTRICT perm, float *FVM_RESTRICT divb,
-    const int *FVM_RESTRICT clist) {
-  corr_cell_dev<R>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, tlast, volp, Wrec, tau, fcon, fcode, U, dU, stepdU, counters, perm, divb, clist, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
-}
-
 // ---- compute_pvel (MPI/compute_pvel.cpp:5-52) -----------------------------
-__device__ __forceinline__ void pvel_body(int i, const Params &P, const unsigned char *FVM_RESTRICT act,
-                       const int *FVM_RESTRICT bnd,
-                       const double *FVM_RESTRICT U, const double *FVM_RESTRICT volp,
+// The mesh velocity of active cell i from its primitives W.
+__device__ __forceinline__ void pvel_state(int i, const Params &P, const double *W, const int *FVM_RESTRICT bnd,
                        const double *FVM_RESTRICT cvol, const double *FVM_RESTRICT ccen,
                        const double *FVM_RESTRICT pos, double *FVM_RESTRICT vel) {
-  if (!(act[i] & A_ACTIVE)) return;
+  double *vo = vel + 3 * (size_t)i;
   if (P.static_mesh) {  // compute_pvel1 hook returning true (MPI/set_problem.cpp:61-72)
-    double *vo = vel + 3 * (size_t)i;
     vo[0] = vo[1] = vo[2] = 0.0;
     return;
   }
-  double W[NF];
-  to_primitive(U + 10 * (size_t)i, volp[i], W);
   double v[3] = {W[VELX], W[VELY], W[VELZ]};
   const double B2 = W[BX] * W[BX] + W[BY] * W[BY] + W[BZ] * W[BZ];
   const double cs2 = (P.gamma * pressure(P, W) + B2) / W[DENS];
@@ -1452,8 +1415,81 @@ __device__ __forceinline__ void pvel_body(int i, const Params &P, const unsigned
     v[0] += d3[0] * f; v[1] += d3[1] * f; v[2] += d3[2] * f;
     if (bnd[i] != NO_BOUNDARY) v[0] = v[1] = v[2] = 0.0;
   }
-  double *vo = vel + 3 * (size_t)i;
   vo[0] = v[0]; vo[1] = v[1]; vo[2] = v[2];
+}
+__device__ __forceinline__ void pvel_body(int i, const Params &P, const unsigned char *FVM_RESTRICT act,
+                       const int *FVM_RESTRICT bnd,
+                       const double *FVM_RESTRICT U, const double *FVM_RESTRICT volp,
+                       const double *FVM_RESTRICT cvol, const double *FVM_RESTRICT ccen,
+                       const double *FVM_RESTRICT pos, double *FVM_RESTRICT vel) {
+  if (!(act[i] & A_ACTIVE)) return;
+  double W[NF];
+  if (!P.static_mesh) to_primitive(U + 10 * (size_t)i, volp[i], W);
+  pvel_state(i, P, W, bnd, cvol, ccen, pos, vel);
+}
+
+// One thread per cell; in partial steps a fixed grid strides over the
+// involved-cell list (clist, count ninv) instead of every cell.
+template <typename R>
+__device__ __forceinline__ void corr_cell_dev(int n, Params P, const Sched *FVM_RESTRICT S,
+    const int *FVM_RESTRICT off, const int2 *FVM_RESTRICT lfj, const int2 *FVM_RESTRICT s12,
+    const double *FVM_RESTRICT cvol, const unsigned char *FVM_RESTRICT act, const int *FVM_RESTRICT bnd,
+    const double *FVM_RESTRICT pos, const double *FVM_RESTRICT tlast, double *FVM_RESTRICT volp,
+    const R *FVM_RESTRICT Wrec, const R *FVM_RESTRICT tau,
+    const R *FVM_RESTRICT fcon, const unsigned char *FVM_RESTRICT fcode,
+    double *FVM_RESTRICT U, double *FVM_RESTRICT dU, double *FVM_RESTRICT stepdU,
+    unsigned long long *FVM_RESTRICT counters, const int *FVM_RESTRICT perm, float *FVM_RESTRICT divb,
+    const int *FVM_RESTRICT clist, const double *FVM_RESTRICT ccen, double *FVM_RESTRICT vel,
+    R *FVM_RESTRICT Wst, int gt0_, int gnt_) {
+  const double t_global = S->t_global;
+  const int cnt = clist ? S->ninv : n;
+  const bool lst = clist && cnt != n;  // every cell involved: the list is the identity
+  for (int t = gt0_; t < cnt; t += gnt_) {
+    const int c = lst ? clist[t] : perm[t];
+    corr_cell_body<R>(c, t_global, P, off, lfj, cvol, act, bnd, pos, tlast, volp, Wrec, tau, fcon, fcode, U, dU,
+                      stepdU, counters, divb);
+    // When a whole step runs (Wst not null), compute_pvel and the primitives
+    // of distribute_fluid_update_data of the same cell: its own updated state,
+    // which no later stage changes, in one conversion.
+    const unsigned char ac = act[c];
+    if (Wst && (ac & (A_ACTIVE | A_LNGB))) {
+      double u[NF], W[NF];
+      load_n<double, NF>(U + 10 * (size_t)c, u);
+      to_primitive(u, volp[c], W);
+      R w[NF];
+#pragma unroll
+      for (int k = 0; k < NF; k++) w[k] = R(W[k]);
+      store_n<R, NF>(Wst + 10 * (size_t)c, w);
+      if (ac & A_ACTIVE) pvel_state(c, P, W, bnd, cvol, ccen, pos, vel);
+    }
+  }
+}
+template <typename R>
+__global__ void __launch_bounds__(128) k_corr_cell(int n, Params P, const Sched *FVM_RESTRICT S,
+    const int *FVM_RESTRICT off, const int2 *FVM_RESTRICT lfj, const int2 *FVM_RESTRICT s12,
+    const double *FVM_RESTRICT cvol, const unsigned char *FVM_RESTRICT act, const int *FVM_RESTRICT bnd,
+    const double *FVM_RESTRICT pos, const double *FVM_RESTRICT tlast, double *FVM_RESTRICT volp,
+    const R *FVM_RESTRICT Wrec, const R *FVM_RESTRICT tau,
+    const R *FVM_RESTRICT fcon, const unsigned char *FVM_RESTRICT fcode,
+    double *FVM_RESTRICT U, double *FVM_RESTRICT dU, double *FVM_RESTRICT stepdU,
+    unsigned long long *FVM_RESTRICT counters, const int *FVM_RESTRICT perm, float *FVM_RESTRICT divb,
+    const int *FVM_RESTRICT clist, const double *FVM_RESTRICT ccen, double *FVM_RESTRICT vel,
+    R *FVM_RESTRICT Wst) {
+  corr_cell_dev<R>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, tlast, volp, Wrec, tau, fcon, fcode, U, dU, stepdU, counters, perm, divb, clist, ccen, vel, Wst, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+// The same for global steps, with more resident blocks.
+template <typename R>
+__global__ void __launch_bounds__(128, FVM_CORR_CELL_MINB(R)) k_corr_cell_g(int n, Params P, const Sched *FVM_RESTRICT S,
+    const int *FVM_RESTRICT off, const int2 *FVM_RESTRICT lfj, const int2 *FVM_RESTRICT s12,
+    const double *FVM_RESTRICT cvol, const unsigned char *FVM_RESTRICT act, const int *FVM_RESTRICT bnd,
+    const double *FVM_RESTRICT pos, const double *FVM_RESTRICT tlast, double *FVM_RESTRICT volp,
+    const R *FVM_RESTRICT Wrec, const R *FVM_RESTRICT tau,
+    const R *FVM_RESTRICT fcon, const unsigned char *FVM_RESTRICT fcode,
+    double *FVM_RESTRICT U, double *FVM_RESTRICT dU, double *FVM_RESTRICT stepdU,
+    unsigned long long *FVM_RESTRICT counters, const int *FVM_RESTRICT perm, float *FVM_RESTRICT divb,
+    const int *FVM_RESTRICT clist, const double *FVM_RESTRICT ccen, double *FVM_RESTRICT vel,
+    R *FVM_RESTRICT Wst) {
+  corr_cell_dev<R>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, tlast, volp, Wrec, tau, fcon, fcode, U, dU, stepdU, counters, perm, divb, clist, ccen, vel, Wst, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 // Every cell, or in partial steps the involved-cell list.
@@ -1573,18 +1609,37 @@ __device__ __forceinline__ void timestep_group(Params P, const int *FVM_RESTRICT
   if ((threadIdx.x & 31) == 0 && vmin < FVM_HUGE) atomic_min_pos(dmin, vmin);
 }
 
+// Also starts the step's adjust_timesteps over from nothing: its counters and
+// flags, and (partial steps: work not null) its marks and work lists, cleared
+// for the involved cells only: every mark, work list and replay write of the
+// step lands on one of them, and every reader walks them only.
 __global__ void k_timestep(int n, Params P, const int *FVM_RESTRICT off, const int2 *FVM_RESTRICT lfj,
                            const unsigned char *FVM_RESTRICT act,
                            const int *FVM_RESTRICT bnd, const double *FVM_RESTRICT U,
                            const double *FVM_RESTRICT volp, const double *FVM_RESTRICT vel,
                            const double *FVM_RESTRICT pos, const double *FVM_RESTRICT tlast,
                            const double *FVM_RESTRICT tend, double *FVM_RESTRICT dtl,
-                           double *FVM_RESTRICT dmin, const int *FVM_RESTRICT clist, const int *FVM_RESTRICT ninv) {
+                           Sched *FVM_RESTRICT S, const int *FVM_RESTRICT clist, int *FVM_RESTRICT aflag,
+                           unsigned char *FVM_RESTRICT hash, unsigned char *FVM_RESTRICT act0,
+                           unsigned char *FVM_RESTRICT work) {
   // one thread per cell: every lane of a group would repeat the cell's own
   // terms (a cube root among them), and on a full step that costs more than
   // the shorter face walk gains (0.26 -> 0.69 ms on the 128^3 blast)
   const int gt = blockIdx.x * blockDim.x + threadIdx.x, gn = gridDim.x * blockDim.x;
-  timestep_group<1>(P, off, lfj, act, bnd, U, volp, vel, pos, tlast, tend, dtl, dmin, clist, clist ? *ninv : 0, 0,
+  if (gt < 4) S->iscal[4 + gt] = 0;
+  if (gt < 8) aflag[gt] = 0;
+  const int ninv = clist ? S->ninv : 0;
+  if (work) {
+    const bool lst = ninv != n;  // every cell involved: the list is the identity
+    for (int t = gt; t < ninv; t += gn) {
+      const int i = lst ? clist[t] : t;
+      hash[i] = 0;
+      act0[i] = 0;
+      work[i] = 0;
+      work[(size_t)n + i] = 0;
+    }
+  }
+  timestep_group<1>(P, off, lfj, act, bnd, U, volp, vel, pos, tlast, tend, dtl, &S->dtmin, clist, ninv, 0,
                     0xffffffffu, gt, gn, n);
 }
 
@@ -1975,24 +2030,6 @@ __global__ void k_adjust_replay(int n, int kparam, const int *FVM_RESTRICT off, 
                                blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, ulist, *ucount);
 }
 
-// A partial step's adjust_timesteps work arrays, cleared for its involved
-// cells only: every mark, work list and replay write of the step lands on
-// one of them, and every reader walks them only (the replays through their
-// list, the sequential sweep's compaction).
-__global__ void k_adjust_clear(int n, const int *FVM_RESTRICT clist, const int *FVM_RESTRICT ninv,
-                               unsigned char *FVM_RESTRICT hash, unsigned char *FVM_RESTRICT act0,
-                               unsigned char *FVM_RESTRICT work) {
-  const int cnt = *ninv;
-  const bool lst = cnt != n;  // every cell involved: the list is the identity
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < cnt; t += gridDim.x * blockDim.x) {
-    const int i = lst ? clist[t] : t;
-    hash[i] = 0;
-    act0[i] = 0;
-    work[i] = 0;
-    work[(size_t)n + i] = 0;
-  }
-}
-
 // In a captured step the replays run as the body of a conditional WHILE
 // node: after replay k this single thread stops the loop once replay k
 // changed nothing (settled) or ADJ_ITERS replays have run, and advances k.
@@ -2080,6 +2117,20 @@ __device__ __forceinline__ void rungs_body(int i, double t_global, int min_rung,
   }
 }
 
+// distribute_fluid_update_data: primitives of the updated state
+template <typename R>
+__device__ __forceinline__ void wst_body(int i, const unsigned char *FVM_RESTRICT act,
+                                         const double *FVM_RESTRICT U, const double *FVM_RESTRICT volp,
+                                         R *FVM_RESTRICT Wst) {
+  if (!(act[i] & (A_ACTIVE | A_LNGB))) return;
+  double u[NF], W[NF];
+  load_n<double, NF>(U + 10 * (size_t)i, u);
+  to_primitive(u, volp[i], W);
+  R w[NF];
+#pragma unroll
+  for (int k = 0; k < NF; k++) w[k] = R(W[k]);
+  store_n<R, NF>(Wst + 10 * (size_t)i, w);
+}
 // Every cell, or in partial steps the involved-cell list.
 template <typename R>
 __device__ __forceinline__ void rungs_dev(int n, Params P, const Sched *FVM_RESTRICT S, int shared,
@@ -2106,20 +2157,6 @@ __global__ void k_rungs(int n, Params P, const Sched *FVM_RESTRICT S, int shared
   rungs_dev<R>(n, P, S, shared, act, hash, dtl, dmin, rung, tlast, tend, Wrec, iscal, vel, opos, ovel, clist, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
-// distribute_fluid_update_data: primitives of the updated state
-template <typename R>
-__device__ __forceinline__ void wst_body(int i, const unsigned char *FVM_RESTRICT act,
-                                         const double *FVM_RESTRICT U, const double *FVM_RESTRICT volp,
-                                         R *FVM_RESTRICT Wst) {
-  if (!(act[i] & (A_ACTIVE | A_LNGB))) return;
-  double u[NF], W[NF];
-  load_n<double, NF>(U + 10 * (size_t)i, u);
-  to_primitive(u, volp[i], W);
-  R w[NF];
-#pragma unroll
-  for (int k = 0; k < NF; k++) w[k] = R(W[k]);
-  store_n<R, NF>(Wst + 10 * (size_t)i, w);
-}
 template <typename R>
 __device__ __forceinline__ void wst_dev(int n, const unsigned char *FVM_RESTRICT act, const double *FVM_RESTRICT U,
                       const double *FVM_RESTRICT volp, R *FVM_RESTRICT Wst, const int *FVM_RESTRICT clist,
@@ -2544,8 +2581,10 @@ __global__ void k_sched_begin(Params P, Sched *S) {
   S->inc[1] = 0;
 }
 
-__global__ void k_sched_end(Sched *S, int n) {
-  S->mnmx_ok = S->iscal[1] == n;
+// The step's end in the scheduler's counters.
+__device__ __forceinline__ void sched_end(Sched *S, int n) {
+  S->mnmx_ok = S->ff_all = S->iscal[1] == n;
+  S->ff_count = S->iscal[3];
   S->nactive_total += (unsigned long long)S->iscal[1];
   S->nfaces_total += (unsigned long long)S->iscal[3];
   S->steps += 1;
@@ -2554,7 +2593,7 @@ __global__ void k_sched_end(Sched *S, int n) {
 __global__ void k_sched_set(Params P, Sched *S, unsigned long long tsysU, int reset_err) {
   S->tsysU = S->tprevU = tsysU;
   S->t_global = P.dt_tick * (double)tsysU;
-  S->mnmx_ok = 0;  // the state was replaced
+  S->mnmx_ok = S->ff_all = 0;  // the state was replaced
   if (reset_err) {
     S->min_rung = 0;
     S->iscal[2] = 0;
@@ -2575,8 +2614,9 @@ __device__ __forceinline__ void maxrung_dev(int n, const int *FVM_RESTRICT rung,
     atomicMax(out, r);
   }
 }
-__global__ void k_maxrung(int n, const int *FVM_RESTRICT rung, int *FVM_RESTRICT out) {
-  maxrung_dev(n, rung, out, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+__global__ void k_maxrung(int n, const int *FVM_RESTRICT rung, Sched *FVM_RESTRICT S, int end) {
+  if (end && blockIdx.x == 0 && threadIdx.x == 0) sched_end(S, n);  // of a step
+  maxrung_dev(n, rung, &S->iscal[0], blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 // (V / (4 pi / 3))^(1/3) per cell, for Params::hcell.

@@ -196,7 +196,7 @@ struct fvm_ctx {
   // fvm_step_host: the copy stream and the events that order its copies
   // against the stage kernels (created on first use)
   cudaStream_t cpy = nullptr;
-  cudaEvent_t hev[5] = {};
+  cudaEvent_t hev[4] = {};
   unsigned *gbar = nullptr;    // its grid barrier
   int *gerr = nullptr;         // its error bits
   std::string err;
@@ -569,10 +569,12 @@ static int read_sched(fvm_ctx *c) {
   return 0;
 }
 
-// Rung maximum over all cells into S->iscal[0] (the next step's max_rung).
-static int enqueue_maxrung(fvm_ctx *c) {
-  CK(cudaMemsetAsync(&c->d.S->iscal[0], 0, sizeof(int), c->st));
-  k_maxrung<<<smin(nblk(c->n, 256), 4 * c->sms), 256, 0, c->st>>>(c->n, c->d.rung, &c->d.S->iscal[0]);
+// Rung maximum over all cells into S->iscal[0] (the next step's max_rung); at
+// the end of a step (end) k_sched_begin has zeroed it, and the scheduler's
+// counters are closed too.
+static int enqueue_maxrung(fvm_ctx *c, int end) {
+  if (!end) CK(cudaMemsetAsync(&c->d.S->iscal[0], 0, sizeof(int), c->st));
+  k_maxrung<<<smin(nblk(c->n, 256), 4 * c->sms), 256, 0, c->st>>>(c->n, c->d.rung, c->d.S, end);
   LAUNCH_CHECK();
   return 0;
 }
@@ -593,6 +595,8 @@ static int enq_positions(fvm_ctx *c, const double *pos, const int *bnd) {
   BULK(k_link_recon<R><<<nblk(n, 256), 256, 0, c->st>>>(n, c->P, d.off, d.lfj, d.geo, d.dr1, d.dr2, (R *)d.lrw,
                                                         (R *)d.lrd, (R *)d.lld));
   LAUNCH_CHECK();
+  // the boundary codes may have changed: the face flags are made anew
+  CK(cudaMemsetAsync(&d.S->ff_all, 0, sizeof(int), c->st));
   c->have_geom = true;
   return 0;
 }
@@ -721,7 +725,7 @@ int fvm_set_state(fvm_ctx *c, const double *vel, const double *tlast, const doub
   CK(cudaMemcpyAsync(c->d.volp, c->d.cvol, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
   k_sched_set<<<1, 1, 0, s>>>(c->P, c->d.S, tsys_ticks, 0);
   LAUNCH_CHECK();
-  int rc = enqueue_maxrung(c);
+  int rc = enqueue_maxrung(c, 0);
   if (rc) return rc;
   c->have_state = true;
   rc = read_sched(c);
@@ -736,7 +740,7 @@ static int enq_lists_meshwide(fvm_ctx *c) {
   Dev &d = c->d;
   // partial steps: blocks of CB faces, whose counts start the face compaction
   k_faceflags<<<nblk(c->nf, CB), CB, 0, c->st>>>(c->nf, d.s12, d.act, d.bnd, d.fflag, &d.S->iscal[3], d.fcode,
-                                                 d.fcode2, c->use_flist ? d.fbcount : nullptr);
+                                                 d.fcode2, c->use_flist ? d.fbcount : nullptr, d.S, c->n);
   LAUNCH_CHECK();
   if (c->use_flist) {
     const int nb = (int)((c->nf + CB - 1) / CB);
@@ -877,8 +881,8 @@ static int enq_begin(fvm_ctx *c) {
 }
 
 // The staged limiter, instantiation MINB (resident blocks per SM).  A partial
-// step launches it on a grid of resident blocks (it returns at once unless
-// every cell is active); a global step on one block per cell block.
+// step launches it on a grid of resident blocks, a global step on one block
+// per cell block.
 extern "C++" {
 template <typename R, int MINB>
 static int limiter_st_launch(fvm_ctx *c) {
@@ -896,7 +900,7 @@ static int limiter_st_launch(fvm_ctx *c) {
   const long long grid = c->use_flist ? std::min<long long>(ncb, (long long)MINB * c->sms) : ncb;
   k_limiter_st<R, KH, MINB><<<(unsigned)grid, 128, limiter_stage_bytes<R, KH>(), c->st>>>(
       c->n, c->P, d.S, d.off, d.lnk, d.lfj, d.s12, d.geo, d.dr1, d.fflag, d.act, d.tlast, (const R *)d.Wrec,
-      (R *)d.tau, (R *)d.fst, d.perm, (const R *)d.mnmx, d.mz, c->use_flist, (const R *)d.lld);
+      (R *)d.tau, (R *)d.fst, d.perm, (const R *)d.mnmx, d.mz, c->use_flist ? d.clist : nullptr, (const R *)d.lld);
   return 0;
 }
 }  // extern "C++"
@@ -905,27 +909,22 @@ static int enq_limiter(fvm_ctx *c) {
   Dev &d = c->d;
   kt_begin(c, KT_LIMITER);
   static_assert(FVM_CELL_PERM == 0, "the staged limiter maps threads to consecutive cells");
-  // Global steps: the staged limiter when the autotuner picked it, else the
-  // per-thread one.  Partial steps launch both: the staged one (one block per
-  // CST cells) works only in a step where every cell is active, the list one
-  // (on a fixed grid) only in the others.
-  const bool staged = c->tune.lim_staged != 0;
-  if (staged) {
+  // The staged limiter when the autotuner picked it (partial steps choose
+  // between its staging and the list on the device), else the per-thread one.
+  if (c->tune.lim_staged != 0) {
     BULK(({
       const int rc = c->use_flist ? limiter_st_launch<R, CellTune<R>::MINB_LIM>(c)
                                   : limiter_st_launch<R, CellTune<R>::MINB_LIM_G>(c);
       if (rc) return rc;
     }));
-    LAUNCH_CHECK();
-  }
-  if (!staged || c->use_flist) {
+  } else {
     const int bs = c->tune.bs_cell2;
 #define LIMITER_LIST(MB)                                                                                       \
   BULK(k_limiter<R, CellTune<R>::KH_LIM, MB>                                                                  \
        <<<sgrid(c, (long long)(10 / CellTune<R>::KH_LIM) * c->n, bs), bs, 0, c->st>>>(                         \
            c->n, c->P, d.S, d.off, d.lnk, d.lfj, d.s12, d.geo, d.dr1, d.fflag, d.act, d.tlast, (const R *)d.Wrec, \
            (R *)d.tau, (R *)d.fst, d.perm, (const R *)d.mnmx, d.mz, c->use_flist ? d.clist : nullptr,          \
-           staged && c->use_flist, (const R *)d.lld))
+           (const R *)d.lld))
     if (c->use_flist) LIMITER_LIST(CellTune<R>::MINB_LIM);
     else LIMITER_LIST(CellTune<R>::MINB_LIM_G);
 #undef LIMITER_LIST
@@ -965,14 +964,16 @@ static int enq_corr_flux(fvm_ctx *c) {
   return 0;
 }
 
-static int enq_corr_cell(fvm_ctx *c) {
+// The cells of compute_update; for a whole step also compute_pvel and the
+// primitives of distribute_fluid_update_data.
+static int enq_corr_cell(fvm_ctx *c, bool whole) {
   Dev &d = c->d;
   kt_begin(c, KT_CORR_CELL);
 #define CORR_CELL(K)                                                                                           \
   BULK(K<R><<<sgrid(c, c->n, c->tune.bs_cell), c->tune.bs_cell, 0, c->st>>>(                                   \
       c->n, c->P, d.S, d.off, d.lfj, d.s12, d.cvol, d.act, d.bnd, d.pos, d.tlast, d.volp, (const R *)d.Wrec,     \
       (const R *)d.tau, (const R *)d.fcon, d.fcode, d.U, d.dU, d.stepdU, d.counters, d.perm, d.divb,            \
-      c->use_flist ? d.clist : nullptr))
+      c->use_flist ? d.clist : nullptr, d.ccen, d.vel, whole ? (R *)d.Wst : nullptr))
   if (c->use_flist || !c->fp32) CORR_CELL(k_corr_cell);
   else CORR_CELL(k_corr_cell_g);  // an FP32 global step: more resident blocks
 #undef CORR_CELL
@@ -982,9 +983,9 @@ static int enq_corr_cell(fvm_ctx *c) {
 }
 
 // compute_update: the face fluxes, then the cells.
-static int enq_update(fvm_ctx *c) {
+static int enq_update(fvm_ctx *c, bool whole) {
   const int rc = enq_corr_flux(c);
-  return rc ? rc : enq_corr_cell(c);
+  return rc ? rc : enq_corr_cell(c, whole);
 }
 
 static int enq_pvel(fvm_ctx *c) {
@@ -1003,7 +1004,8 @@ static int enq_timesteps(fvm_ctx *c, int shared) {
   kt_begin(c, KT_TIMESTEP);
   const int *cl = c->use_flist ? d.clist : nullptr;  // partial steps: the involved cells only
   k_timestep<<<sgrid(c, n, 128), 128, 0, c->st>>>(n, c->P, d.off, d.lfj, d.act, d.bnd, d.U, d.volp, d.vel,
-                                                  d.pos, d.tlast, d.tend, d.dtl, &d.S->dtmin, cl, &d.S->ninv);
+                                                  d.pos, d.tlast, d.tend, d.dtl, d.S, cl, d.aflag, d.hash, d.act0,
+                                                  shared ? nullptr : d.awork);
   LAUNCH_CHECK();
   if (c->reduce) {  // the minimum over ranks (MPI/compute_timestep.cpp:101)
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1019,13 +1021,9 @@ static int enq_timesteps(fvm_ctx *c, int shared) {
   if (!shared) {
     k_halve<<<sgrid(c, n, 256), 256, 0, c->st>>>(n, d.act, &d.S->dtmin, d.dtl, cl, &d.S->ninv);
     LAUNCH_CHECK();
-    CK(cudaMemsetAsync(&d.S->iscal[4], 0, 4 * sizeof(int), c->st));
-    k_adjust_clear<<<sgrid(c, n, 256), 256, 0, c->st>>>(n, cl, &d.S->ninv, d.hash, d.act0, d.awork);
-    LAUNCH_CHECK();
     k_adjust_mark<<<sgrid(c, 8LL * n, 128), 128, 0, c->st>>>(n, d.off, d.lfj, d.act, d.bnd, d.dtl, d.hash,
                                                       &d.S->iscal[4], d.act0, d.awork, cl, &d.S->ninv);
     LAUNCH_CHECK();
-    CK(cudaMemsetAsync(d.aflag, 0, 8 * sizeof(int), c->st));
     k_adjust_init<<<sgrid(c, n, 256), 256, 0, c->st>>>(n, d.off, d.lfj, d.act, &d.S->iscal[4], d.dtl, d.dt0,
                                                       d.rdv, d.wrv, d.aflag, cl, &d.S->ninv);
     LAUNCH_CHECK();
@@ -1157,14 +1155,12 @@ static int enq_recon(fvm_ctx *c) {
 static int enq_end(fvm_ctx *c, int shared) {
   Dev &d = c->d;
   kt_begin(c, KT_SYNC);
-  int rc = enqueue_maxrung(c);
+  int rc = enqueue_maxrung(c, 1);
   if (rc) return rc;
   if (shared) {
     k_shared_sync<<<nblk(c->n, 256), 256, 0, c->st>>>(c->n, c->P, d.S, d.act, d.S->iscal, d.rung, d.tend);
     LAUNCH_CHECK();
   }
-  k_sched_end<<<1, 1, 0, c->st>>>(d.S, c->n);
-  LAUNCH_CHECK();
   kt_end(c, KT_SYNC);
   return 0;
 }
@@ -1174,10 +1170,8 @@ static int enq_end(fvm_ctx *c, int shared) {
 static int enq_stages(fvm_ctx *c, int shared) {
   int rc;
   if ((rc = enq_limiter(c))) return rc;
-  if ((rc = enq_update(c))) return rc;
-  if ((rc = enq_pvel(c))) return rc;
+  if ((rc = enq_update(c, true))) return rc;  // with compute_pvel and the updated primitives
   if ((rc = enq_timesteps(c, shared))) return rc;
-  if ((rc = enq_collect(c))) return rc;
   if ((rc = enq_update0(c))) return rc;
   return enq_recon(c);
 }
@@ -1313,7 +1307,7 @@ int fvm_begin_step(fvm_ctx *c) {
 }
 
 int fvm_slope_limiter(fvm_ctx *c) { STEP_GUARD("fvm_slope_limiter"); return enq_limiter(c); }
-int fvm_compute_update(fvm_ctx *c) { STEP_GUARD("fvm_compute_update"); return enq_update(c); }
+int fvm_compute_update(fvm_ctx *c) { STEP_GUARD("fvm_compute_update"); return enq_update(c, false); }
 int fvm_compute_pvel(fvm_ctx *c) { STEP_GUARD("fvm_compute_pvel"); return enq_pvel(c); }
 
 int fvm_compute_timesteps(fvm_ctx *c, int shared, double *dt_min_out) {
@@ -1377,7 +1371,7 @@ int fvm_step(fvm_ctx *c, int shared) {
 // and then overwritten in place, with the copies of U and dU on a second
 // stream overlapping the stage kernels: in before the compute_update cell
 // pass needs them, out as soon as that pass has finished them (the later
-// stages do not write U or dU), then the velocities after compute_pvel and
+// stages do not write U or dU) with the velocities, which it sets too, then
 // tlast after the rungs; rung, tend and the reconstruction after the step.
 // Always the stage kernels.
 int fvm_step_host(fvm_ctx *c, int shared, unsigned long long tsys_ticks, double *vel, double *tlast, double *tend,
@@ -1418,7 +1412,7 @@ int fvm_step_host(fvm_ctx *c, int shared, unsigned long long tsys_ticks, double 
   CK(cudaMemcpyAsync(d.volp, d.cvol, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
   k_sched_set<<<1, 1, 0, st>>>(c->P, d.S, tsys_ticks, 0);
   LAUNCH_CHECK();
-  int rc = enqueue_maxrung(c);
+  int rc = enqueue_maxrung(c, 0);
   if (rc) return rc;
   // U and dU on the copy stream once the early inputs are in (the two would
   // only share the link), while the step's first stages run
@@ -1434,20 +1428,16 @@ int fvm_step_host(fvm_ctx *c, int shared, unsigned long long tsys_ticks, double 
   if (c->learn_mode == 1) CK(cudaStreamWaitEvent(st, c->hev[1], 0));
   if ((rc = enq_corr_flux(c))) return rc;
   CK(cudaStreamWaitEvent(st, c->hev[1], 0));
-  if ((rc = enq_corr_cell(c))) return rc;
+  if ((rc = enq_corr_cell(c, true))) return rc;  // with compute_pvel and the updated primitives
   CK(cudaEventRecord(c->hev[2], st));
   CK(cudaStreamWaitEvent(cs, c->hev[2], 0));
   CK(cudaMemcpyAsync(U, d.U, 10 * n * sizeof(double), cudaMemcpyDeviceToHost, cs));
   CK(cudaMemcpyAsync(dU, d.dU, 14 * n * sizeof(double), cudaMemcpyDeviceToHost, cs));
-  if ((rc = enq_pvel(c))) return rc;
-  CK(cudaEventRecord(c->hev[3], st));
-  CK(cudaStreamWaitEvent(cs, c->hev[3], 0));
   CK(cudaMemcpyAsync(vel, d.vel, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, cs));
   if ((rc = enq_timesteps(c, shared))) return rc;
-  CK(cudaEventRecord(c->hev[4], st));
-  CK(cudaStreamWaitEvent(cs, c->hev[4], 0));
+  CK(cudaEventRecord(c->hev[3], st));
+  CK(cudaStreamWaitEvent(cs, c->hev[3], 0));
   CK(cudaMemcpyAsync(tlast, d.tlast, n * sizeof(double), cudaMemcpyDeviceToHost, cs));
-  if ((rc = enq_collect(c))) return rc;
   if ((rc = enq_update0(c))) return rc;
   if ((rc = enq_recon(c))) return rc;
   if ((rc = enq_end(c, shared))) return rc;
@@ -2415,6 +2405,7 @@ int fvm_autotune(fvm_ctx *c, int shared, int steps, int *choice) {
     }
     for (int k = 0; k < KT_COUNT; k++) ms_out[k] = c->kt_ms[k];
     if ((r = state_copy(c, sc, false))) return r;
+    CK(cudaMemsetAsync(&c->d.S->ff_all, 0, sizeof(int), c->st));  // the face flags are the trial's
     CK(cudaStreamSynchronize(c->st));
     c->tsysU = tsys0;
     c->t_global = t0;
