@@ -63,8 +63,8 @@ struct Dev {
   int *aflag;               // adjust_timesteps replay flags
   unsigned char *awork;     // adjust_timesteps replay work lists (2 per cell)
   void *mnmx;               // per cell: the reconstruction's neighbour min and max (20 of the bulk type)
-  void *lrw;                // per link: the reconstruction's face weights (6, bulk type)
-  void *lrd;                // per link: the face centroid's offset from the cell (3, bulk type)
+  void *lrw, *lrd;          // per link: the reconstruction's records (ReconLink)
+  double *csum;             // per cell: sums over its faces of n A and of the centroid's offset (6)
   void *lld;                // per link: the limiter's face-side offset dr (3, bulk type)
   unsigned char *mz;        // per cell: the reconstruction met a boundary (the limiter is zero)
   // learned-flux buffers (fvm_set_flux_mode)
@@ -404,6 +404,44 @@ __global__ void k_inc_faces(const int *FVM_RESTRICT off, const int2 *FVM_RESTRIC
   }
 }
 
+// KH consecutive bulk values from p, as 2-wide loads when KH is even: the
+// callers' rows (10 or 50 values per cell, 6 per link) and even offsets then
+// start on 16-byte (FP64) or 8-byte (FP32) boundaries.
+template <typename R> struct Vec2;
+template <> struct Vec2<double> { using T = double2; };
+template <> struct Vec2<float> { using T = float2; };
+template <typename R, int N>
+__device__ __forceinline__ void load_n(const R *FVM_RESTRICT p, R *v) {
+  if constexpr (N % 2 == 0) {
+    using V = typename Vec2<R>::T;
+    const V *p2 = reinterpret_cast<const V *>(p);
+#pragma unroll
+    for (int h = 0; h < N / 2; h++) { const V x = p2[h]; v[2 * h] = x.x; v[2 * h + 1] = x.y; }
+  } else {
+#pragma unroll
+    for (int k = 0; k < N; k++) v[k] = p[k];
+  }
+}
+
+template <typename R, int N>
+__device__ __forceinline__ void store_n(R *FVM_RESTRICT p, const R *v) {
+  if constexpr (N % 2 == 0) {
+    using V = typename Vec2<R>::T;
+    V *p2 = reinterpret_cast<V *>(p);
+#pragma unroll
+    for (int h = 0; h < N / 2; h++) { V x; x.x = v[2 * h]; x.y = v[2 * h + 1]; p2[h] = x; }
+  } else {
+#pragma unroll
+    for (int k = 0; k < N; k++) p[k] = v[k];
+  }
+}
+
+// Four values as one 256-bit load (32-byte aligned) of data constant in the
+// launch.
+__device__ __forceinline__ void load4c(const double *p, double *v) {
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+}
+
 // Face offsets used by every face loop, computed once per generator layout:
 //   dr1 = centroid - x_s1 (the reference's dri, MPI/compute_update.cpp:136)
 //         with w = dri . n (dsh, :164)
@@ -442,14 +480,19 @@ __device__ __forceinline__ void wrap3(const Params &P, double *d) {
 
 // Geometry of one face side for the reconstruction
 // (MPI/compute_reconstruction.cpp:70-138): the min-image offset d of the face
-// centroid, the normal oriented along it and the normal distance dsh.
+// centroid, the normal oriented along it and the normal distance dsh, rounded
+// as the reference's operations are (no contraction).
+__device__ __forceinline__ double dot3_rn(const double *a, const double *b) {
+  return __dadd_rn(__dadd_rn(__dmul_rn(a[0], b[0]), __dmul_rn(a[1], b[1])), __dmul_rn(a[2], b[2]));
+}
 __device__ __forceinline__ void recon_geom(const Params &P, bool own, const double4 &g, const double4 &o4, double *d,
                                            double *nrm, double &dsh) {
   d[0] = o4.x; d[1] = o4.y; d[2] = o4.z;
   if (own) wrap3(P, d);
-  const double sgn = (d[0] * g.x + d[1] * g.y + d[2] * g.z) < 0.0 ? -1.0 : 1.0;
+  const double n[3] = {g.x, g.y, g.z};
+  const double sgn = dot3_rn(d, n) < 0.0 ? -1.0 : 1.0;
   nrm[0] = g.x * sgn; nrm[1] = g.y * sgn; nrm[2] = g.z * sgn;
-  dsh = d[0] * nrm[0] + d[1] * nrm[1] + d[2] * nrm[2];
+  dsh = dot3_rn(d, nrm);
 }
 // A / (2 dsh), the face weight of the gradient.
 __device__ __forceinline__ double recon_ia(const double4 &g, double dsh) {
@@ -457,18 +500,43 @@ __device__ __forceinline__ double recon_ia(const double4 &g, double dsh) {
 }
 
 // The reconstruction's per-link records, computed once per mesh (the mesh is
-// fixed while it is installed).  The face term of the gradient,
-// ((wj + wi) dsh n + (wj - wi) (d - dsh n)) A / (2 dsh), becomes
-// (wj + wi) a + (wj - wi) b with a = dsh n A/(2 dsh), b = (d - dsh n) A/(2 dsh)
-// (lrw: a then b), and the limiter pass reads the min-image offset d (lrd).
-// The face loops then do no geometry, no division and one dependent load.
+// fixed while it is installed), so that its face loops do no geometry and no
+// division.  d is the min-image offset of the face centroid, ia = A / (2 dsh);
+// the face term of the gradient is
+// ((wj + wi) dsh n + (wj - wi) (d - dsh n)) ia.
+//
+// FP64 (lrw: d, ia): the term is (wj - wi) ia d plus wi (2 dsh n ia), whose
+// second factor, n A, sums over the cell's faces to a constant of the mesh
+// (csum; round-off on a closed cell).  One 32-byte record serves both face
+// loops (separate factors of wj + wi and wj - wi, and d, took 72 bytes), and
+// the loop's rounding errors are of the size of the differences, not of the
+// states.  The constant multiplies the states themselves, the same way in
+// every step, so it is summed in double-double from the factors dsh n and ia
+// as the reference rounds them: summed in double, the psi of a 32^3 Alfven
+// wave drifted 1.6e-12 from the oracle in ten steps, with this sum 0.9e-12
+// (separate factors: 0.7e-12).  128^3 blast: 1.78 -> 1.41 ms.
+//
+// FP32: (wj + wi) a + (wj - wi) b with a = dsh n ia, b = (d - dsh n) ia (lrw: a,
+// b), and d (lrd).  The FP64 form would round differently, and single
+// precision shows that in the limiter of nearly flat states.  (One 32-byte
+// record with the neighbour in it, and d padded to 16 bytes, measured 1.06
+// against 1.03 ms: two threads per cell are not bound by their loads.)
+template <typename R> struct ReconLink;
+template <> struct ReconLink<double> { static constexpr int NW = 4, ND = 0; };
+template <> struct ReconLink<float> { static constexpr int NW = 6, ND = 3; };
+__device__ __forceinline__ void dd_add(double &hi, double &lo, double x) {
+  const double s = __dadd_rn(hi, x), b = __dadd_rn(s, -hi);
+  lo = __dadd_rn(lo, __dadd_rn(__dadd_rn(hi, -__dadd_rn(s, -b)), __dadd_rn(x, -b)));
+  hi = s;
+}
 template <typename R>
 __global__ void k_link_recon(int n, Params P, const int *FVM_RESTRICT off, const int2 *FVM_RESTRICT lfj,
                              const double4 *FVM_RESTRICT geo, const double4 *FVM_RESTRICT dr1,
                              const double4 *FVM_RESTRICT dr2, R *FVM_RESTRICT lrw, R *FVM_RESTRICT lrd,
-                             R *FVM_RESTRICT lld) {
+                             double *FVM_RESTRICT csum, R *FVM_RESTRICT lld) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
+  double sum[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, low[3] = {0.0, 0.0, 0.0};
   for (int q = off[c]; q < off[c + 1]; q++) {
     const int2 fj = lfj[q];
     const bool own = fj.y >= 0;
@@ -476,12 +544,24 @@ __global__ void k_link_recon(int n, Params P, const int *FVM_RESTRICT off, const
     double d[3], nrm[3], dsh;
     recon_geom(P, own, g, own ? dr1[fj.x] : dr2[fj.x], d, nrm, dsh);
     const double ia = recon_ia(g, dsh);
-    R *w = lrw + 6 * (size_t)q, *o = lrd + 3 * (size_t)q;
+    if constexpr (sizeof(R) == 8) {
+      const R w[4] = {d[0], d[1], d[2], ia};
+      store_n<R, 4>(lrw + 4 * (size_t)q, w);
+    } else {
+      R *w = lrw + 6 * (size_t)q, *o = lrd + 3 * (size_t)q;
+#pragma unroll
+      for (int a = 0; a < 3; a++) {
+        w[a] = R(nrm[a] * dsh * ia);
+        w[3 + a] = R((d[a] - nrm[a] * dsh) * ia);
+        o[a] = R(d[a]);
+      }
+    }
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-      w[a] = R(nrm[a] * dsh * ia);
-      w[3 + a] = R((d[a] - nrm[a] * dsh) * ia);
-      o[a] = R(d[a]);
+      const double f = 2.0 * __dmul_rn(nrm[a], dsh), p = __dmul_rn(f, ia);
+      dd_add(sum[a], low[a], p);
+      low[a] += fma(f, ia, -p);  // the product's rounding error
+      sum[3 + a] = sum[3 + a] + double(R(d[a]));
     }
     // the limiter's offset of this side: dri for s1, dri - 2 dsh n for s2
     // (MPI/compute_update.cpp:157-212; dr1 unwrapped, as the limiter uses it)
@@ -490,6 +570,9 @@ __global__ void k_link_recon(int n, Params P, const int *FVM_RESTRICT off, const
     R *l3 = lld + 3 * (size_t)q;
     l3[0] = R(e.x - g.x * dsl); l3[1] = R(e.y - g.y * dsl); l3[2] = R(e.z - g.z * dsl);
   }
+#pragma unroll
+  for (int a = 0; a < 3; a++) sum[a] = __dadd_rn(sum[a], low[a]);
+  store_n<double, 6>(csum + 6 * (size_t)c, sum);
 }
 
 // ---- slope_limiter (MPI/compute_reconstruction.cpp:201-602) --------------
@@ -528,38 +611,6 @@ template <> struct CellTune<float> {
   static constexpr int KH_LIM = 2, MINB_LIM = 8, KH_REC = 5, MINB_REC = 6;
   static constexpr int MINB_LIM_G = FVM_LIMITER_MINB_F, MINB_REC_G = FVM_RECON_MINB_F;
 };
-
-// KH consecutive bulk values from p, as 2-wide loads when KH is even: the
-// callers' rows (10 or 50 values per cell, 6 per link) and even offsets then
-// start on 16-byte (FP64) or 8-byte (FP32) boundaries.
-template <typename R> struct Vec2;
-template <> struct Vec2<double> { using T = double2; };
-template <> struct Vec2<float> { using T = float2; };
-template <typename R, int N>
-__device__ __forceinline__ void load_n(const R *FVM_RESTRICT p, R *v) {
-  if constexpr (N % 2 == 0) {
-    using V = typename Vec2<R>::T;
-    const V *p2 = reinterpret_cast<const V *>(p);
-#pragma unroll
-    for (int h = 0; h < N / 2; h++) { const V x = p2[h]; v[2 * h] = x.x; v[2 * h + 1] = x.y; }
-  } else {
-#pragma unroll
-    for (int k = 0; k < N; k++) v[k] = p[k];
-  }
-}
-
-template <typename R, int N>
-__device__ __forceinline__ void store_n(R *FVM_RESTRICT p, const R *v) {
-  if constexpr (N % 2 == 0) {
-    using V = typename Vec2<R>::T;
-    V *p2 = reinterpret_cast<V *>(p);
-#pragma unroll
-    for (int h = 0; h < N / 2; h++) { V x; x.x = v[2 * h]; x.y = v[2 * h + 1]; p2[h] = x; }
-  } else {
-#pragma unroll
-    for (int k = 0; k < N; k++) p[k] = v[k];
-  }
-}
 
 // A face's 14 contributions as seven 2-wide stores (records of 112 bytes in
 // FP64, 56 in FP32).
@@ -2388,8 +2439,8 @@ template <typename R, int KH>
 __device__ __forceinline__ void recon_body(int c, int k0, const Params &P, const int *FVM_RESTRICT off,
     const int2 *FVM_RESTRICT lfj, const double *FVM_RESTRICT cvol, const unsigned char *FVM_RESTRICT act,
     const int *FVM_RESTRICT bnd, const R *FVM_RESTRICT Wst, const int *FVM_RESTRICT rung, R *FVM_RESTRICT Wrec,
-    R *FVM_RESTRICT mnmx, unsigned char *FVM_RESTRICT mz, const R *FVM_RESTRICT lrw, const R *FVM_RESTRICT lrd,
-    const unsigned char *FVM_RESTRICT bnb) {
+    R *FVM_RESTRICT mnmx, unsigned char *FVM_RESTRICT mz, const R *FVM_RESTRICT lrw,
+    const R *FVM_RESTRICT lrd, const double *FVM_RESTRICT csum, const unsigned char *FVM_RESTRICT bnb) {
   if (!(act[c] & A_ACTIVE)) return;
   R *r = Wrec + 50 * (size_t)c + k0;
   const R *wsi = Wst + 10 * (size_t)c + k0;
@@ -2408,28 +2459,32 @@ __device__ __forceinline__ void recon_body(int c, int k0, const Params &P, const
   // a boundary neighbour zeroes the reconstruction (its min/max are then unused)
   const bool zero = bnb[c] != 0;
   const int qe = zero ? q0 : q1;
-  auto face_term = [&](const R *w6, const R *Wj) {
-#pragma unroll
-    for (int k = 0; k < KH; k++) {
-      const R wj = Wj[k];
-      const R sum = wj + Wi[k];
-      const R diff = wj - Wi[k];
-      mn[k] = smin(mn[k], diff);
-      mx[k] = smax(mx[k], diff);
-      Wx[k] += sum * w6[0] + diff * w6[3];
-      Wy[k] += sum * w6[1] + diff * w6[4];
-      Wz[k] += sum * w6[2] + diff * w6[5];
-    }
-  };
   FVM_CELL_LOOP
   for (int q = q0; q < qe; q++) {
     const int2 fj = lfj[q];
     const int j = fj.y >= 0 ? fj.y : ~fj.y;
-    R w6[6];
-    load_n<R, 6>(lrw + 6 * (size_t)q, w6);
-    R Wj[KH];
+    R w[ReconLink<R>::NW], Wj[KH];
+    if constexpr (sizeof(R) == 8) load4c(lrw + 4 * (size_t)q, w);
+    else load_n<R, 6>(lrw + 6 * (size_t)q, w);
     load_n<R, KH>(Wst + 10 * (size_t)j + k0, Wj);
-    face_term(w6, Wj);
+#pragma unroll
+    for (int k = 0; k < KH; k++) {
+      const R wj = Wj[k];
+      const R diff = wj - Wi[k];
+      mn[k] = smin(mn[k], diff);
+      mx[k] = smax(mx[k], diff);
+      if constexpr (sizeof(R) == 8) {
+        const R e = diff * w[3];
+        Wx[k] += e * w[0];
+        Wy[k] += e * w[1];
+        Wz[k] += e * w[2];
+      } else {
+        const R sum = wj + Wi[k];
+        Wx[k] += sum * w[0] + diff * w[3];
+        Wy[k] += sum * w[1] + diff * w[4];
+        Wz[k] += sum * w[2] + diff * w[5];
+      }
+    }
   }
   // the next step's limiter pass 1 (neighbour min/max of the same states)
   {
@@ -2443,18 +2498,24 @@ __device__ __forceinline__ void recon_body(int c, int k0, const Params &P, const
     return;
   }
   const R invV = R(1.0 / cvol[c]);
+  const double *cs = csum + 6 * (size_t)c;
   R ln[KH], lq[KH], thr[KH];
 #pragma unroll
   for (int k = 0; k < KH; k++) {
-    Wx[k] *= invV; Wy[k] *= invV; Wz[k] *= invV; ln[k] = R(2); lq[k] = R(1);
+    if constexpr (sizeof(R) == 8) {
+      Wx[k] += Wi[k] * cs[0];
+      Wy[k] += Wi[k] * cs[1];
+      Wz[k] += Wi[k] * cs[2];
+    }
+    Wx[k] *= invV; Wy[k] *= invV; Wz[k] *= invV;
+    ln[k] = R(2); lq[k] = R(1);
     thr[k] = limiter_thr(mn[k], mx[k]);
   }
-  double sc[3] = {0.0, 0.0, 0.0};
   FVM_CELL_LOOP
   for (int q = q0; q < q1; q++) {
-    const R *o3 = lrd + 3 * (size_t)q;
-    const R dd[3] = {o3[0], o3[1], o3[2]};
-    sc[0] = sc[0] + double(dd[0]); sc[1] = sc[1] + double(dd[1]); sc[2] = sc[2] + double(dd[2]);
+    R dd[4];
+    if constexpr (sizeof(R) == 8) load4c(lrw + 4 * (size_t)q, dd);
+    else load_n<R, 3>(lrd + 3 * (size_t)q, dd);
 #pragma unroll
     for (int k = 0; k < KH; k++) {
       const R dWx = Wx[k] * dd[0] + Wy[k] * dd[1] + Wz[k] * dd[2];
@@ -2470,7 +2531,7 @@ __device__ __forceinline__ void recon_body(int c, int k0, const Params &P, const
   }
   if (k0 == 0) {  // density positivity for the *-state (MPI/compute_reconstruction.cpp:179-197)
     const R sum_dt = R(get_dt(P, rung[c]));
-    const R dWx = Wx[0] * R(sc[0]) + Wy[0] * R(sc[1]) + Wz[0] * R(sc[2]);
+    const R dWx = Wx[0] * R(cs[3]) + Wy[0] * R(cs[4]) + Wz[0] * R(cs[5]);
     const R dWp = dWx + tt[0] * sum_dt;
     const R dW = smax(dWx, dWp);
     if (dW > R(0)) {
@@ -2492,7 +2553,7 @@ __device__ __forceinline__ void recon_dev(int n, Params P, const Sched *FVM_REST
     const double *FVM_RESTRICT cvol, const unsigned char *FVM_RESTRICT act, const int *FVM_RESTRICT bnd,
     const R *FVM_RESTRICT Wst, const int *FVM_RESTRICT rung, R *FVM_RESTRICT Wrec, const int *FVM_RESTRICT perm,
     R *FVM_RESTRICT mnmx, unsigned char *FVM_RESTRICT mz, const R *FVM_RESTRICT lrw,
-    const R *FVM_RESTRICT lrd, const int *FVM_RESTRICT clist, const unsigned char *FVM_RESTRICT bnb, int gt0_, int gnt_) {
+    const R *FVM_RESTRICT lrd, const double *FVM_RESTRICT csum, const int *FVM_RESTRICT clist, const unsigned char *FVM_RESTRICT bnb, int gt0_, int gnt_) {
   constexpr int TPC = 10 / KH;
   const long long cnt = (long long)TPC * (clist ? S->ninv : n);
   const bool lst = clist && S->ninv != n;  // every cell involved: the list is the identity
@@ -2500,7 +2561,7 @@ __device__ __forceinline__ void recon_dev(int n, Params P, const Sched *FVM_REST
        t += (long long)gnt_) {
     const int u = (int)(t / TPC);
     recon_body<R, KH>(lst ? clist[u] : perm[u], (int)(t % TPC) * KH, P, off, lfj, cvol, act, bnd, Wst, rung, Wrec,
-                      mnmx, mz, lrw, lrd, bnb);
+                      mnmx, mz, lrw, lrd, csum, bnb);
   }
 }
 template <typename R, int KH, int MINB>
@@ -2509,8 +2570,8 @@ __global__ void __launch_bounds__(128, MINB) k_recon(int n, Params P, const Sche
     const double *FVM_RESTRICT cvol, const unsigned char *FVM_RESTRICT act, const int *FVM_RESTRICT bnd,
     const R *FVM_RESTRICT Wst, const int *FVM_RESTRICT rung, R *FVM_RESTRICT Wrec, const int *FVM_RESTRICT perm,
     R *FVM_RESTRICT mnmx, unsigned char *FVM_RESTRICT mz, const R *FVM_RESTRICT lrw,
-    const R *FVM_RESTRICT lrd, const int *FVM_RESTRICT clist, const unsigned char *FVM_RESTRICT bnb) {
-  recon_dev<R, KH, MINB>(n, P, S, off, lfj, cvol, act, bnd, Wst, rung, Wrec, perm, mnmx, mz, lrw, lrd, clist, bnb, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    const R *FVM_RESTRICT lrd, const double *FVM_RESTRICT csum, const int *FVM_RESTRICT clist, const unsigned char *FVM_RESTRICT bnb) {
+  recon_dev<R, KH, MINB>(n, P, S, off, lfj, cvol, act, bnd, Wst, rung, Wrec, perm, mnmx, mz, lrw, lrd, csum, clist, bnb, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 // Per link (a cell's entry in its face list, i.e. one side of a face), in the

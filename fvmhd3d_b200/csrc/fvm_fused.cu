@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(128, FVM_FLUX_MINB(R)) k_rung_step(FusedStep a
   FVM_GRID_SYNC();
   recon_dev<R, CellTune<R>::KH_REC, CellTune<R>::MINB_REC>(n, P, S, d.off, d.lfj, d.cvol, d.act, d.bnd,
                                                            (const R *)d.Wst, d.rung, (R *)d.Wrec, d.perm,
-                                                           (R *)d.mnmx, d.mz, (const R *)d.lrw, (const R *)d.lrd,
+                                                           (R *)d.mnmx, d.mz, (const R *)d.lrw, (const R *)d.lrd, d.csum,
                                                            d.clist, d.bnb, gt, gn);
   if (gt == 0) S->fused_steps += 1;
 #undef FVM_GRID_SYNC

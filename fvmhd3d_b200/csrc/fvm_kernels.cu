@@ -393,8 +393,9 @@ static int alloc_mesh(fvm_ctx *c, long long ncell, long long nface, long long nl
   rc |= dalloc(c, &d.aflag, 8);
   rc |= dalloc(c, &d.awork, 2 * (size_t)ncell);
   rc |= dalloc_bytes(c, &d.mnmx, 20 * c->rb * (size_t)ncell); rc |= dalloc(c, &d.mz, ncell);
-  rc |= dalloc_bytes(c, &d.lrw, 6 * c->rb * (size_t)nl);
-  rc |= dalloc_bytes(c, &d.lrd, 3 * c->rb * (size_t)nl);
+  BULK(rc |= dalloc_bytes(c, &d.lrw, ReconLink<R>::NW * sizeof(R) * (size_t)nl);
+       rc |= dalloc_bytes(c, &d.lrd, ReconLink<R>::ND * sizeof(R) * (size_t)nl));
+  rc |= dalloc(c, &d.csum, 6 * (size_t)ncell);
   rc |= dalloc_bytes(c, &d.lld, 3 * c->rb * (size_t)nl);
   rc |= dalloc(c, &d.alist, ncell);
   rc |= dalloc(c, &d.pos, 3 * (size_t)ncell); rc |= dalloc(c, &d.vel, 3 * (size_t)ncell);
@@ -593,7 +594,7 @@ static int enq_positions(fvm_ctx *c, const double *pos, const int *bnd) {
   k_face_geom<<<nblk(c->nf, 256), 256, 0, c->st>>>(c->nf, c->P, d.s12, d.geo, d.cen, d.pos, d.dr1, d.dr2);
   LAUNCH_CHECK();
   BULK(k_link_recon<R><<<nblk(n, 256), 256, 0, c->st>>>(n, c->P, d.off, d.lfj, d.geo, d.dr1, d.dr2, (R *)d.lrw,
-                                                        (R *)d.lrd, (R *)d.lld));
+                                                        (R *)d.lrd, d.csum, (R *)d.lld));
   LAUNCH_CHECK();
   // the boundary codes may have changed: the face flags are made anew
   CK(cudaMemsetAsync(&d.S->ff_all, 0, sizeof(int), c->st));
@@ -1143,7 +1144,7 @@ static int enq_recon(fvm_ctx *c) {
   BULK(k_recon<R, CellTune<R>::KH_REC, MB>                                                                     \
        <<<sgrid(c, (long long)(10 / CellTune<R>::KH_REC) * c->n, c->tune.bs_cell2), c->tune.bs_cell2, 0, c->st>>>( \
            c->n, c->P, d.S, d.off, d.lfj, d.cvol, d.act, d.bnd, (const R *)d.Wst, d.rung, (R *)d.Wrec, d.perm,   \
-           (R *)d.mnmx, d.mz, (const R *)d.lrw, (const R *)d.lrd, c->use_flist ? d.clist : nullptr, d.bnb))
+           (R *)d.mnmx, d.mz, (const R *)d.lrw, (const R *)d.lrd, d.csum, c->use_flist ? d.clist : nullptr, d.bnb))
   if (c->use_flist) RECON(CellTune<R>::MINB_REC);
   else RECON(CellTune<R>::MINB_REC_G);  // a global step: more resident blocks (FP32)
 #undef RECON
