@@ -593,20 +593,20 @@ template <> struct CellTune<double> {
 #define FVM_RECON_MINB_D 8
 #endif
 #ifndef FVM_LIMITER_MINB_D
-#define FVM_LIMITER_MINB_D 6
+#define FVM_LIMITER_MINB_D 7
 #endif
   static constexpr int KH_LIM = 2, MINB_LIM = FVM_LIMITER_MINB_D, KH_REC = 2, MINB_REC = FVM_RECON_MINB_D;
   static constexpr int MINB_LIM_G = MINB_LIM, MINB_REC_G = MINB_REC;  // global steps: the same
 };
 template <> struct CellTune<float> {
 // global steps: 8 blocks for the reconstruction (64 registers, a few
-// spills) and 10 for the limiter (46) beat 6 and 8 (128^3 blast: 1.085 ->
-// 1.027 ms and 0.915 -> 0.886 ms)
+// spills) beat 6 (128^3 blast: 1.085 -> 1.027 ms) and 12 for the limiter beat
+// 10 (0.88 -> 0.845 ms, now that its staging leaves room for them)
 #ifndef FVM_RECON_MINB_F
 #define FVM_RECON_MINB_F 8
 #endif
 #ifndef FVM_LIMITER_MINB_F
-#define FVM_LIMITER_MINB_F 10
+#define FVM_LIMITER_MINB_F 12
 #endif
   static constexpr int KH_LIM = 2, MINB_LIM = 8, KH_REC = 5, MINB_REC = 6;
   static constexpr int MINB_LIM_G = FVM_LIMITER_MINB_F, MINB_REC_G = FVM_RECON_MINB_F;
@@ -867,15 +867,21 @@ __device__ __forceinline__ void limiter_group(int i, int k0, int gl, unsigned gm
 }
 
 // Staged limiter: a block's CST cells (TPC threads each) first compute the
-// per-face records of passes 2 and 3 (the side's offset dr, the two time
-// offsets, the face and its flags) for all their faces together, into shared
-// memory, so the face loops read no global memory but the cell's own record.
-// Used when the first pass is reused (every cell steps) and the block's faces
-// fit (LCAP); otherwise the block runs limiter_thread.
+// per-face records of passes 2 and 3 (the side's offset dr, its time offset,
+// the face and its flags) for all their faces together, into shared memory, so
+// the face loops read no global memory but the cell's own record.  Used when
+// the first pass is reused (every cell steps) and the block's faces fit
+// (LCAP); otherwise the block runs limiter_thread.  A cell's records start at
+// a slot congruent to its number modulo 8: the cells of a warp, at the same
+// face of their lists, then read different banks (packed starts, often 16
+// faces apart, took three passes per read on average: 41% of the L1 data pipe).
+// That and one time offset per record instead of two (they are equal) leave
+// room for more blocks per SM: 7 instead of 6 in FP64 (128^3 blast 1.54 ->
+// 1.46 ms; 8 spill: 1.65), 12 instead of 10 in FP32 (0.91 -> 0.845).
 template <int KH> __host__ __device__ constexpr int limiter_cst() { return 128 / (10 / KH); }  // cells per block
-template <int KH> __host__ __device__ constexpr int limiter_lcap() { return 22 * limiter_cst<KH>(); }
+template <int KH> __host__ __device__ constexpr int limiter_lcap() { return 26 * limiter_cst<KH>(); }
 template <typename R, int KH>
-constexpr int limiter_stage_bytes() { return limiter_lcap<KH>() * (5 * (int)sizeof(R) + 4); }
+constexpr int limiter_stage_bytes() { return limiter_lcap<KH>() * (4 * (int)sizeof(R) + 4); }
 
 // One block's CST cells (cell block cb); called by every thread of the block.
 template <typename R, int KH>
@@ -891,12 +897,29 @@ __device__ __forceinline__ void limiter_st_block(int cb, int n, bool reuse, doub
   const int c0 = cb * CST;
   const int c1 = c0 + CST < n ? c0 + CST : n;
   const int L0 = off[c0], nL = off[c1] - L0;
-  const bool staged = reuse && nL <= LCAP;  // uniform over the block
-  R *sdx = reinterpret_cast<R *>(lsm), *sdy = sdx + LCAP, *sdz = sdy + LCAP, *st2 = sdz + LCAP, *st3 = st2 + LCAP;
-  int *sfk = reinterpret_cast<int *>(st3 + LCAP);
+  R *sdx = reinterpret_cast<R *>(lsm), *sdy = sdx + LCAP, *sdz = sdy + LCAP, *sdt = sdz + LCAP;
+  int *sfk = reinterpret_cast<int *>(sdt + LCAP);
+  static_assert(CST < 32, "one warp lays the cells out");
+  bool staged = reuse;  // uniform over the block
   if (staged) {
-    for (int k = tid; k <= c1 - c0; k += blockDim.x) soff[k] = off[c0 + k] - L0;
+    int *sbase = soff + CST + 1;
+    if (tid < 32) {
+      const int o = off[c0 + min(tid, c1 - c0)] - L0;
+      const int cnt = __shfl_down_sync(0xffffffffu, o, 1) - o;  // of cell tid
+      int end = tid < c1 - c0 ? cnt + ((1 - cnt) & 7) : 0;  // its slots: 1 modulo 8
+      for (int k = 1; k < 32; k <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, end, k);
+        if (tid >= k) end += y;
+      }
+      if (tid <= CST) soff[tid] = o;
+      if (tid < CST) sbase[tid + 1] = end;
+      if (tid == 0) sbase[0] = 0;
+    }
     __syncthreads();
+    staged = sbase[c1 - c0] <= LCAP;
+  }
+  if (staged) {
+    const int *sbase = soff + CST + 1;
     for (int l = tid; l < nL; l += blockDim.x) {
       int lo = 0, hi = c1 - c0;  // soff[lo] <= l < soff[hi]
       while (hi - lo > 1) {
@@ -910,14 +933,13 @@ __device__ __forceinline__ void limiter_st_block(int cb, int n, bool reuse, doub
       const double ti = tlast[c0 + lo], tj = tlast[own ? fj.y : ~fj.y];
       const double dtI = t_global - (own ? ti : tj), dtJ = t_global - (own ? tj : ti);
       const double dth = 0.5 * smin(dtI, dtJ);
-      const double dt = smin(dtI, dtJ);
       const R *l3 = lld + 3 * (size_t)(L0 + l);
-      sdx[l] = l3[0];
-      sdy[l] = l3[1];
-      sdz[l] = l3[2];
-      st2[l] = R(own ? dtI - dth : dtJ - dth);
-      st3[l] = R(own ? dtI - 0.5 * dt : dtJ - 0.5 * dt);
-      sfk[l] = (f << 3) | ((ff & FF_ACTIVE) ? 1 : 0) | ((ff & (FF_BND1 | FF_BND2)) ? 2 : 0) | (own ? 4 : 0);
+      const int m = sbase[lo] + l - soff[lo];
+      sdx[m] = l3[0];
+      sdy[m] = l3[1];
+      sdz[m] = l3[2];
+      sdt[m] = R(own ? dtI - dth : dtJ - dth);
+      sfk[m] = (f << 3) | ((ff & FF_ACTIVE) ? 1 : 0) | ((ff & (FF_BND1 | FF_BND2)) ? 2 : 0) | (own ? 4 : 0);
     }
   }
   __syncthreads();
@@ -938,7 +960,7 @@ __device__ __forceinline__ void limiter_st_block(int cb, int n, bool reuse, doub
     mn[k] = mm[k]; mx[k] = mm[10 + k]; ln[k] = R(2); lq[k] = R(1); wi[k] = ri[k];
   }
   const bool zero = mz[i] != 0;
-  const int q0 = soff[cl], q1 = soff[cl + 1];
+  const int q0 = soff[CST + 1 + cl], q1 = q0 + soff[cl + 1] - soff[cl];
   R *to = tau + 10 * (size_t)i + k0;
   if (zero) {
 #pragma unroll
@@ -952,7 +974,7 @@ __device__ __forceinline__ void limiter_st_block(int cb, int n, bool reuse, doub
     }
     for (int l = q0; l < q1; l++) {
       if (!(sfk[l] & 1)) continue;
-      const R d0 = sdx[l], d1 = sdy[l], d2 = sdz[l], dtt = st2[l];
+      const R d0 = sdx[l], d1 = sdy[l], d2 = sdz[l], dtt = sdt[l];
 #pragma unroll
       for (int k = 0; k < KH; k++) {
         const R dWx = gx[k] * d0 + gy[k] * d1 + gz[k] * d2;
@@ -970,7 +992,7 @@ __device__ __forceinline__ void limiter_st_block(int cb, int n, bool reuse, doub
   for (int l = q0; l < q1; l++) {
     const int fk = sfk[l];
     if (!(fk & 1) || (fk & 2)) continue;
-    const R d0 = sdx[l], d1 = sdy[l], d2 = sdz[l], dtt = st3[l];
+    const R d0 = sdx[l], d1 = sdy[l], d2 = sdz[l], dtt = sdt[l];
     R o[KH];
 #pragma unroll
     for (int k = 0; k < KH; k++) o[k] = wi[k] + ((gx[k] * d0 + gy[k] * d1 + gz[k] * d2) + gt[k] * dtt);
@@ -1025,7 +1047,7 @@ __global__ void __launch_bounds__(128, MINB) k_limiter_st(int n, Params P, const
     const R *FVM_RESTRICT mnmx, const unsigned char *FVM_RESTRICT mz, const int *FVM_RESTRICT clist, const R *FVM_RESTRICT lld) {
   constexpr int CST = limiter_cst<KH>();
   extern __shared__ __align__(16) unsigned char lsm[];
-  __shared__ int soff[CST + 1];
+  __shared__ int soff[2 * (CST + 1)];  // the cells' first links, and their first slots
   if (clist && S->iscal[1] != n) {
     limiter_dev<R, KH, MINB>(n, P, S, off, lnk, lfj, s12, geo, dr1, fflag, act, tlast, Wrec, tau, fst, perm, mnmx, mz,
                              clist, lld, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
