@@ -1921,111 +1921,58 @@ int fvm_mlp_get_weights(fvm_ctx *c, float *params) {
   return 0;
 }
 
-// ---- training: forward + backward of one batch of `rows` rows ---------------
-// Largest K split of a training product (the weight gradients: M, N <= 128,
-// K = batch rows), and the partial tiles it needs.
-constexpr int kMaxSplit = 64;
-
+// ---- training ----------------------------------------------------------------
+// One batch's work space: the pairs, the loss weights, the weight operands, the
+// CTAs' sums and, for training, Adam's moments, in one allocation.
 struct MlpWork {
-  int rows = 0;
-  float *X, *T, *Z1, *Z2, *Z3, *Z4, *A1, *A2, *A3, *G, *dA, *dB, *grad, *loss, *wt, *m, *v, *part;
+  int ncta = 0, per = 0;  // CTAs of k_fwd_bwd and the rows of each
+  float *X, *T, *wt, *m, *v, *grad, *hist, *part, *dz;
+  unsigned char *img;
   void *base = nullptr;
 };
 
-static int mlp_work(fvm_ctx *c, MlpWork &w, int rows) {
+// Room for n pairs and `hist` losses; batches of `rows` rows.
+static int mlp_work(fvm_ctx *c, MlpWork &w, long long n, int rows, int hist) {
   using namespace mlp;
-  const size_t npart = (size_t)kMaxSplit * NH * NH;  // split-K partial tiles of the weight gradients
-  const size_t nf = (size_t)rows * (NIN + NOUT + 3 * NH + NOUT + 3 * NH + NOUT + 2 * NH) + 3 * (size_t)NPARAM + 1 + NOUT +
-                    npart;
+  // rows in chunks of 64, at most 64 CTAs of at least two chunks each (the
+  // order of the weight gradients' sums)
+  const int chunks = (rows + 63) / 64, want = chunks >= 4 ? std::min(64, chunks / 2) : 1;
+  w.per = 64 * ((chunks + want - 1) / want);
+  w.ncta = (rows + w.per - 1) / w.per;
+  auto pad = [](size_t k) { return (k + 63) & ~(size_t)63; };  // regions start 256-byte aligned
+  const size_t sizes[] = {pad((size_t)n * NIN), pad((size_t)n * NOUT), pad(NOUT), pad(NPARAM), pad(NPARAM), pad(NPARAM),
+                          pad(hist), pad((size_t)w.ncta * mlpt::PART), pad((size_t)rows * (3 * NH + NOUT)),
+                          pad(mlpt::I_BYTES / 4)};
+  size_t nf = 0;
+  for (size_t k : sizes) nf += k;
   CK(cudaMallocAsync(&w.base, nf * sizeof(float), c->st));
-  CK(cudaMemsetAsync(w.base, 0, nf * sizeof(float), c->st));
   float *p = (float *)w.base;
-  auto take = [&](size_t k) { float *q = p; p += k; return q; };
-  w.rows = rows;
-  w.X = take((size_t)rows * NIN); w.T = take((size_t)rows * NOUT);
-  w.Z1 = take((size_t)rows * NH); w.Z2 = take((size_t)rows * NH); w.Z3 = take((size_t)rows * NH);
-  w.Z4 = take((size_t)rows * NOUT);
-  w.A1 = take((size_t)rows * NH); w.A2 = take((size_t)rows * NH); w.A3 = take((size_t)rows * NH);
-  w.G = take((size_t)rows * NOUT); w.dA = take((size_t)rows * NH); w.dB = take((size_t)rows * NH);
-  w.grad = take(NPARAM); w.m = take(NPARAM); w.v = take(NPARAM); w.loss = take(1); w.wt = take(NOUT);
-  w.part = take(npart);
-  // the tensor-core product's shared memory, set once per device
+  float **at[] = {&w.X, &w.T, &w.wt, &w.m, &w.v, &w.grad, &w.hist, &w.part, &w.dz};
+  for (int k = 0; k < 9; k++) { *at[k] = p; p += sizes[k]; }
+  w.img = (unsigned char *)p;
+  // Adam's moments start at zero, and so do the operands' padding rows
+  CK(cudaMemsetAsync(w.m, 0, 2 * sizes[3] * sizeof(float), c->st));
+  CK(cudaMemsetAsync(w.img, 0, mlpt::I_BYTES, c->st));
+  mlpt::k_operands<<<nblk(NPARAM, 256), 256, 0, c->st>>>(c->mlp_param, w.img);
+  LAUNCH_CHECK();
+  // the kernel's shared memory, set once per device
   static bool attr[kMaxDevices] = {};
   if (c->device < 0 || c->device >= kMaxDevices) { c->err = "device index out of range"; return FVM_EINVAL; }
   if (!attr[c->device]) {
-    CK(cudaFuncSetAttribute(mlpt::k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, mlpt::TC_SMEM));
+    CK(cudaFuncSetAttribute(mlpt::k_fwd_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, mlpt::S_BYTES));
+    CK(cudaFuncSetAttribute(mlpt::k_update, cudaFuncAttributeMaxDynamicSharedMemorySize, mlpt::U_BYTES));
     attr[c->device] = true;
   }
   return 0;
 }
 
-// C = A B on the tensor cores (mlpt::k_gemm_tc).  Products with one output
-// tile and a long K are split over up to kMaxSplit CTAs of at least two
-// chunks each and summed in split order.
-static void gemm(fvm_ctx *c, const MlpWork &w, int M, int N, int K, const float *A, long long sam, long long sak,
-                 const float *B, long long sbk, long long sbn, float *C, int ldc) {
-  cudaStream_t s = c->st;
-  const int tiles_m = (M + mlpt::TM - 1) / mlpt::TM, tiles_n = (N + mlpt::TN - 1) / mlpt::TN;
-  const int nchunk = (K + mlpt::TK - 1) / mlpt::TK;
-  int nsplit = 1, cps = nchunk;
-  if (tiles_m * tiles_n == 1 && nchunk >= 4) {
-    nsplit = std::min(kMaxSplit, nchunk / 2);
-    cps = (nchunk + nsplit - 1) / nsplit;
-    nsplit = (nchunk + cps - 1) / cps;
-  }
-  dim3 grid(tiles_n, tiles_m, nsplit);
-  mlpt::k_gemm_tc<<<grid, 128, mlpt::TC_SMEM, s>>>(M, N, K, A, sam, sak, B, sbk, sbn, C, ldc, 0, cps, w.part,
-                                                   c->mlp_err);
-  if (nsplit > 1) mlpt::k_splitk_sum<<<(M * N + 255) / 256, 256, 0, s>>>(M, N, nsplit, w.part, C, ldc, 0);
-}
-
-// Loss (added to *w.loss) and gradient (w.grad) of the batch in w.X / w.T at
-// the parameters P.
-static int mlp_fwd_bwd(fvm_ctx *c, MlpWork &w, const float *P) {
-  using namespace mlp;
-  const int B = w.rows;
-  cudaStream_t s = c->st;
-  const float *W1 = P, *b1 = W1 + NH * NIN, *W2 = b1 + NH, *b2 = W2 + NH * NH, *W3 = b2 + NH, *b3 = W3 + NH * NH,
-              *W4 = b3 + NH, *b4 = W4 + NOUT * NH;
-  float *g = w.grad;
-  float *gW1 = g, *gb1 = gW1 + NH * NIN, *gW2 = gb1 + NH, *gb2 = gW2 + NH * NH, *gW3 = gb2 + NH,
-        *gb3 = gW3 + NH * NH, *gW4 = gb3 + NH, *gb4 = gW4 + NOUT * NH;
-  const long long nh = (long long)B * NH;
-  const unsigned eb = (unsigned)((nh + 255) / 256);
-  // forward
-  gemm(c, w, B, NH, NIN, w.X, NIN, 1, W1, 1, NIN, w.Z1, NH);
-  mlpt::k_bias_gelu<<<eb, 256, 0, s>>>(B, NH, w.Z1, b1, w.A1);
-  gemm(c, w, B, NH, NH, w.A1, NH, 1, W2, 1, NH, w.Z2, NH);
-  mlpt::k_bias_gelu<<<eb, 256, 0, s>>>(B, NH, w.Z2, b2, w.A2);
-  gemm(c, w, B, NH, NH, w.A2, NH, 1, W3, 1, NH, w.Z3, NH);
-  mlpt::k_bias_gelu<<<eb, 256, 0, s>>>(B, NH, w.Z3, b3, w.A3);
-  gemm(c, w, B, NOUT, NH, w.A3, NH, 1, W4, 1, NH, w.Z4, NOUT);
-  mlpt::k_out_loss<<<(B * NOUT + 255) / 256, 256, 0, s>>>(B, w.Z4, b4, w.T, w.wt, w.G, w.loss);
-  // backward
-  gemm(c, w, NOUT, NH, B, w.G, 1, NOUT, w.A3, NH, 1, gW4, NH);
-  mlpt::k_colsum<<<1, 32, 0, s>>>(B, NOUT, w.G, gb4);
-  gemm(c, w, B, NH, NOUT, w.G, NOUT, 1, W4, NH, 1, w.dA, NH);
-  mlpt::k_gelu_back<<<eb, 256, 0, s>>>(nh, w.dA, w.Z3);
-  gemm(c, w, NH, NH, B, w.dA, 1, NH, w.A2, NH, 1, gW3, NH);
-  mlpt::k_colsum<<<1, NH, 0, s>>>(B, NH, w.dA, gb3);
-  gemm(c, w, B, NH, NH, w.dA, NH, 1, W3, NH, 1, w.dB, NH);
-  mlpt::k_gelu_back<<<eb, 256, 0, s>>>(nh, w.dB, w.Z2);
-  gemm(c, w, NH, NH, B, w.dB, 1, NH, w.A1, NH, 1, gW2, NH);
-  mlpt::k_colsum<<<1, NH, 0, s>>>(B, NH, w.dB, gb2);
-  gemm(c, w, B, NH, NH, w.dB, NH, 1, W2, NH, 1, w.dA, NH);
-  mlpt::k_gelu_back<<<eb, 256, 0, s>>>(nh, w.dA, w.Z1);
-  gemm(c, w, NH, NIN, B, w.dA, 1, NH, w.X, NIN, 1, gW1, NIN);
-  mlpt::k_colsum<<<1, NH, 0, s>>>(B, NH, w.dA, gb1);
-  c->launches += 21;
-  CK(cudaGetLastError());
-  return 0;
-}
-
-static int mlp_set_wt(fvm_ctx *c, MlpWork &w, const float *wt) {
+// The pairs and loss weights from the host (wt may be NULL: 1).
+static int mlp_upload(fvm_ctx *c, MlpWork &w, long long n, const float *X, const float *T, const float *wt) {
   float h[mlp::NOUT];
   for (int k = 0; k < mlp::NOUT; k++) h[k] = wt ? wt[k] : 1.0f;
-  CK(cudaMemcpyAsync(w.wt, h, sizeof(h), cudaMemcpyHostToDevice, c->st));
-  CK(cudaStreamSynchronize(c->st));  // h is on the stack
+  CK(cudaMemcpyAsync(w.wt, h, sizeof(h), cudaMemcpyHostToDevice, c->st));  // pageable: staged before the call returns
+  CK(cudaMemcpyAsync(w.X, X, (size_t)n * mlp::NIN * sizeof(float), cudaMemcpyHostToDevice, c->st));
+  CK(cudaMemcpyAsync(w.T, T, (size_t)n * mlp::NOUT * sizeof(float), cudaMemcpyHostToDevice, c->st));
   return 0;
 }
 
@@ -2034,14 +1981,17 @@ int fvm_mlp_grad(fvm_ctx *c, int n, const float *X, const float *T, const float 
   if (!c->mlp_param) { c->err = "fvm_mlp_grad: no weights"; return FVM_EINVAL; }
   CK(cudaSetDevice(c->device));
   MlpWork w;
-  int rc = mlp_work(c, w, n);
+  int rc = mlp_work(c, w, n, n, 1);
   if (rc) return rc;
-  if ((rc = mlp_set_wt(c, w, wt))) return rc;
-  CK(cudaMemcpyAsync(w.X, X, (size_t)n * mlp::NIN * sizeof(float), cudaMemcpyHostToDevice, c->st));
-  CK(cudaMemcpyAsync(w.T, T, (size_t)n * mlp::NOUT * sizeof(float), cudaMemcpyHostToDevice, c->st));
-  if ((rc = mlp_fwd_bwd(c, w, c->mlp_param))) return rc;
+  if ((rc = mlp_upload(c, w, n, X, T, wt))) return rc;
+  mlpt::k_fwd_bwd<<<w.ncta, mlpt::THREADS, mlpt::S_BYTES, c->st>>>(n, w.per, n, w.X, w.T, 0, 0, 0, c->mlp_param, w.img, w.wt,
+                                                                  w.part, w.dz, c->mlp_err);
+  LAUNCH_CHECK();
+  mlpt::k_update<<<mlpt::UBLOCKS, mlpt::UTHREADS, mlpt::U_BYTES, c->st>>>(n, w.ncta, w.part, w.dz, w.grad, w.hist, nullptr, nullptr, nullptr,
+                                                                nullptr, c->mlp_err, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f);
+  LAUNCH_CHECK();
   CK(cudaMemcpyAsync(grad, w.grad, mlp::NPARAM * sizeof(float), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaMemcpyAsync(loss, w.loss, sizeof(float), cudaMemcpyDeviceToHost, c->st));
+  CK(cudaMemcpyAsync(loss, w.hist, sizeof(float), cudaMemcpyDeviceToHost, c->st));
   int herr = 0;
   CK(cudaMemcpyAsync(&herr, c->mlp_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
   CK(cudaFreeAsync(w.base, c->st));
@@ -2056,38 +2006,28 @@ int fvm_mlp_train(fvm_ctx *c, long long n, const float *X, const float *T, const
   if (!c->mlp_param) { c->err = "fvm_mlp_train: no initial weights"; return FVM_EINVAL; }
   CK(cudaSetDevice(c->device));
   MlpWork w;
-  int rc = mlp_work(c, w, batch);
+  int rc = mlp_work(c, w, n, batch, steps > 0 ? steps : 1);
   if (rc) return rc;
-  if ((rc = mlp_set_wt(c, w, wt))) return rc;
-  float *dX = nullptr, *dT = nullptr, *hist = nullptr;
-  CK(cudaMallocAsync(&dX, (size_t)n * mlp::NIN * sizeof(float), c->st));
-  CK(cudaMallocAsync(&dT, (size_t)n * mlp::NOUT * sizeof(float), c->st));
-  CK(cudaMallocAsync(&hist, (size_t)(steps > 0 ? steps : 1) * sizeof(float), c->st));
-  CK(cudaMemcpyAsync(dX, X, (size_t)n * mlp::NIN * sizeof(float), cudaMemcpyHostToDevice, c->st));
-  CK(cudaMemcpyAsync(dT, T, (size_t)n * mlp::NOUT * sizeof(float), cudaMemcpyHostToDevice, c->st));
+  if ((rc = mlp_upload(c, w, n, X, T, wt))) return rc;
   const float b1 = 0.9f, b2 = 0.999f;
   double p1 = 1.0, p2 = 1.0;
   for (int it = 0; it < steps; it++) {
-    mlpt::k_gather<<<(batch + 127) / 128, 128, 0, c->st>>>(n, dX, dT, batch, seed, it, w.X, w.T);
-    CK(cudaMemsetAsync(w.loss, 0, sizeof(float), c->st));
-    if ((rc = mlp_fwd_bwd(c, w, c->mlp_param))) return rc;
+    mlpt::k_fwd_bwd<<<w.ncta, mlpt::THREADS, mlpt::S_BYTES, c->st>>>(batch, w.per, n, w.X, w.T, 1, seed, it, c->mlp_param, w.img,
+                                                                    w.wt, w.part, w.dz, c->mlp_err);
+    LAUNCH_CHECK();
     p1 *= b1;
     p2 *= b2;
-    mlpt::k_adam<<<(mlp::NPARAM + 255) / 256, 256, 0, c->st>>>(mlp::NPARAM, c->mlp_param, w.grad, w.m, w.v, lr, b1,
-                                                               b2, 1e-8f, (float)(1.0 - p1), (float)(1.0 - p2));
-    CK(cudaMemcpyAsync(hist + it, w.loss, sizeof(float), cudaMemcpyDeviceToDevice, c->st));
-    c->launches += 2;
+    mlpt::k_update<<<mlpt::UBLOCKS, mlpt::UTHREADS, mlpt::U_BYTES, c->st>>>(batch, w.ncta, w.part, w.dz, nullptr, w.hist + it, c->mlp_param, w.m,
+                                                                  w.v, w.img, c->mlp_err, lr, b1, b2, 1e-8f, (float)(1.0 - p1),
+                                                                  (float)(1.0 - p2));
+    LAUNCH_CHECK();
   }
-  CK(cudaGetLastError());
   mlp::k_mlp_pack<<<(mlp::NH * mlp::NH + 255) / 256, 256, 0, c->st>>>(c->mlp_param, c->mlp_img);
   LAUNCH_CHECK();
   if (loss_out && steps > 0)
-    CK(cudaMemcpyAsync(loss_out, hist, (size_t)steps * sizeof(float), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(loss_out, w.hist, (size_t)steps * sizeof(float), cudaMemcpyDeviceToHost, c->st));
   int herr = 0;
   CK(cudaMemcpyAsync(&herr, c->mlp_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaFreeAsync(dX, c->st));
-  CK(cudaFreeAsync(dT, c->st));
-  CK(cudaFreeAsync(hist, c->st));
   CK(cudaFreeAsync(w.base, c->st));
   CK(cudaStreamSynchronize(c->st));
   if (herr & 4) { c->err = "fvm_mlp_train: tensor-core product wait timed out"; return FVM_ECUDA; }
