@@ -89,34 +89,33 @@ struct Dev {
 using namespace fvm;
 
 // Minimum resident 128-thread blocks per SM for the face-flux kernels (caps
-// their registers): 3 (168 registers, FP64) or 4 (128, FP32).
+// their registers at 128).  In FP64 4 against 3 (168 registers) took the
+// corrector pass of the 128^3 blast from 1.30 to 1.21 ms and the predictor's
+// from 1.23 to 1.095 ms; 5 (96 registers, spills) 1.39 and 1.165 ms.
 //
 // FP32 global steps (every cell active) launch their own instantiations of
 // the exact face passes, the compute_update / compute_update0 cell passes,
 // the limiter and the reconstruction, with more resident blocks: the extra
-// warps hide more of the gathers than the spills cost (128^3 blast: exact
-// flux at 6 blocks, 80 registers: corrector 0.85 -> 0.69 ms, predictor
-// 0.80 -> 0.63 ms).  Partial steps keep the instantiations whose bits the
-// persistent rung kernel reproduces: the compiler may contract a multiply
-// and an add differently when the register budget changes, so a kernel
-// compiled to another budget need not give the same last bit.  FP64 keeps
-// one set of instantiations: at 4 blocks its face passes were 7-9% faster,
-// but the 32^3 Alfven wave's reconstruction then drifted from the oracle
-// by 1.18e-12 in ten steps, past the 1e-12 parity bound.
-#ifndef FVM_FLUX_MINB_D
-#define FVM_FLUX_MINB_D 3
+// warps hide more of the gathers than the spills cost (128^3 blast, corrector
+// at 6 blocks, 80 registers: 0.85 -> 0.69 ms; predictor at 7, 72 registers:
+// 0.80 -> 0.61 ms, 0.635 at 6; 8 rounds differently).  Partial steps keep the
+// instantiations whose
+// bits the persistent rung kernel reproduces: the compiler may contract a
+// multiply and an add differently when the register budget changes, so a
+// kernel compiled to another budget need not give the same last bit.  (What
+// the oracle comparison sees of such changes, the rounding of the faces'
+// normal fields, is not left to contraction: dot3_rn.)
+#ifndef FVM_FLUX_MINB
+#define FVM_FLUX_MINB 4
 #endif
-#ifndef FVM_FLUX_MINB_F
-#define FVM_FLUX_MINB_F 4
+#ifndef FVM_GLOBAL_CORR_MINB_F
+#define FVM_GLOBAL_CORR_MINB_F 6
 #endif
-#ifndef FVM_GLOBAL_FLUX_MINB_D
-#define FVM_GLOBAL_FLUX_MINB_D FVM_FLUX_MINB_D
+#ifndef FVM_GLOBAL_PRED_MINB_F
+#define FVM_GLOBAL_PRED_MINB_F 7
 #endif
-#ifndef FVM_GLOBAL_FLUX_MINB_F
-#define FVM_GLOBAL_FLUX_MINB_F 6
-#endif
-#define FVM_FLUX_MINB(R) (sizeof(R) == 4 ? FVM_FLUX_MINB_F : FVM_FLUX_MINB_D)
-#define FVM_GLOBAL_FLUX_MINB(R) (sizeof(R) == 4 ? FVM_GLOBAL_FLUX_MINB_F : FVM_GLOBAL_FLUX_MINB_D)
+#define FVM_GLOBAL_CORR_MINB(R) (sizeof(R) == 4 ? FVM_GLOBAL_CORR_MINB_F : FVM_FLUX_MINB)
+#define FVM_GLOBAL_PRED_MINB(R) (sizeof(R) == 4 ? FVM_GLOBAL_PRED_MINB_F : FVM_FLUX_MINB)
 #ifndef FVM_CELL_LFJ
 #define FVM_CELL_LFJ 1  // cell kernels take (face, neighbour) from the link table instead of s12
 #endif
@@ -442,6 +441,36 @@ __device__ __forceinline__ void load4c(const double *p, double *v) {
   asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
 }
 
+// A double4 of mesh data as one 256-bit load.
+__device__ __forceinline__ double4 load_d4(const double4 *p) {
+  double v[4];
+  load4c(reinterpret_cast<const double *>(p), v);
+  return make_double4(v[0], v[1], v[2], v[3]);
+}
+
+// A face's two extrapolated states, in FP64 as five 256-bit loads (a file whose
+// kernel writes the states too, as the persistent kernel does, defines
+// FVM_COHERENT_STATES; 128^3 corrector 1.36 -> 1.30 ms).  In FP32 as pairs: 128-bit
+// loads measured 0.726 against 0.70 ms.
+__device__ __forceinline__ void load_states(const double *FVM_RESTRICT p, double *a, double *b) {
+  double v[20];
+#pragma unroll
+  for (int k = 0; k < 20; k += 4) {
+#ifdef FVM_COHERENT_STATES
+    const double2 x = *reinterpret_cast<const double2 *>(p + k), y = *reinterpret_cast<const double2 *>(p + k + 2);
+    v[k] = x.x; v[k + 1] = x.y; v[k + 2] = y.x; v[k + 3] = y.y;
+#else
+    load4c(p + k, v + k);
+#endif
+  }
+#pragma unroll
+  for (int k = 0; k < NF; k++) { a[k] = v[k]; b[k] = v[NF + k]; }
+}
+__device__ __forceinline__ void load_states(const float *FVM_RESTRICT p, float *a, float *b) {
+  load_n<float, NF>(p, a);
+  load_n<float, NF>(p + NF, b);
+}
+
 // Face offsets used by every face loop, computed once per generator layout:
 //   dr1 = centroid - x_s1 (the reference's dri, MPI/compute_update.cpp:136)
 //         with w = dri . n (dsh, :164)
@@ -482,17 +511,14 @@ __device__ __forceinline__ void wrap3(const Params &P, double *d) {
 // (MPI/compute_reconstruction.cpp:70-138): the min-image offset d of the face
 // centroid, the normal oriented along it and the normal distance dsh, rounded
 // as the reference's operations are (no contraction).
-__device__ __forceinline__ double dot3_rn(const double *a, const double *b) {
-  return __dadd_rn(__dadd_rn(__dmul_rn(a[0], b[0]), __dmul_rn(a[1], b[1])), __dmul_rn(a[2], b[2]));
-}
 __device__ __forceinline__ void recon_geom(const Params &P, bool own, const double4 &g, const double4 &o4, double *d,
                                            double *nrm, double &dsh) {
   d[0] = o4.x; d[1] = o4.y; d[2] = o4.z;
   if (own) wrap3(P, d);
   const double n[3] = {g.x, g.y, g.z};
-  const double sgn = dot3_rn(d, n) < 0.0 ? -1.0 : 1.0;
+  const double sgn = dot3_rn(d[0], d[1], d[2], n[0], n[1], n[2]) < 0.0 ? -1.0 : 1.0;
   nrm[0] = g.x * sgn; nrm[1] = g.y * sgn; nrm[2] = g.z * sgn;
-  dsh = dot3_rn(d, nrm);
+  dsh = dot3_rn(d[0], d[1], d[2], nrm[0], nrm[1], nrm[2]);
 }
 // A / (2 dsh), the face weight of the gradient.
 __device__ __forceinline__ double recon_ia(const double4 &g, double dsh) {
@@ -1127,13 +1153,9 @@ __device__ __forceinline__ void corr_face(int f, int slot, double t_global, cons
   const unsigned char ff = fflag[f];
   if (!(ff & FF_ACTIVE)) return;  // coded F_OFF with the flags
   const int2 e = s12[f];
-  const double4 g = geo[f], d = dr1[f];
+  const double4 g = load_d4(geo + f), d = load_d4(dr1 + f);
   R Wi[NF], Wj[NF];
-  {  // issued with the face record, before the boundary tests
-    const R *fs = fst + 20 * (size_t)f;
-    load_n<R, NF>(fs, Wi);
-    load_n<R, NF>(fs + 10, Wj);
-  }
+  load_states(fst + 20 * (size_t)f, Wi, Wj);  // issued with the face record, before the boundary tests
   int i = e.x, j = e.y;
   const double area = g.w;
   double nrm[3] = {g.x, g.y, g.z};
@@ -1202,7 +1224,7 @@ __device__ __forceinline__ void corr_flux_dev(int nf, Params P, const Sched *FVM
     corr_face<R, MODE>(t, -1, t_global, P, S, s12, geo, dr1, fflag, bnd, vel, tlast, Wrec, fst, fcon, fcode, lb);
   }
 }
-template <typename R, int MODE, int MB = FVM_FLUX_MINB(R)>
+template <typename R, int MODE, int MB = FVM_FLUX_MINB>
 __global__ void __launch_bounds__(128, MB) k_corr_flux(int nf, Params P, const Sched *FVM_RESTRICT S,
     const int2 *FVM_RESTRICT s12, const double4 *FVM_RESTRICT geo, const double4 *FVM_RESTRICT dr1,
     const unsigned char *FVM_RESTRICT fflag, const int *FVM_RESTRICT bnd, const double *FVM_RESTRICT vel,
@@ -2257,7 +2279,7 @@ __device__ __forceinline__ void pred_face(int f, int slot, const Params &P,
   if (!(ff & FF_ACTIVE)) return;  // coded F_OFF with the flags
   const int2 e = s12[f];
   int i = e.x, j = e.y;
-  const double4 g = geo[f], d = dr1[f];
+  const double4 g = load_d4(geo + f), d = load_d4(dr1 + f);
   const double area = g.w;
   double nrm[3] = {g.x, g.y, g.z};
   double dri[3] = {d.x, d.y, d.z};
@@ -2325,7 +2347,7 @@ __device__ __forceinline__ void pred_flux_dev(int nf, Params P,
     pred_face<R, MODE>(t, -1, P, s12, geo, dr1, fflag, bnd, vel, Wst, fcon, fcode, S, rung, lb);
   }
 }
-template <typename R, int MODE, int MB = FVM_FLUX_MINB(R)>
+template <typename R, int MODE, int MB = FVM_FLUX_MINB>
 __global__ void __launch_bounds__(128, MB) k_pred_flux(int nf, Params P,
     const int2 *FVM_RESTRICT s12, const double4 *FVM_RESTRICT geo, const double4 *FVM_RESTRICT dr1,
     const unsigned char *FVM_RESTRICT fflag, const int *FVM_RESTRICT bnd,

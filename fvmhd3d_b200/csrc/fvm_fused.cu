@@ -13,6 +13,7 @@
 // FVM_RESTRICT empty: a stage here reads what earlier stages of the same
 // launch wrote on other SMs, so nothing is promised read-only.
 #define FVM_RESTRICT
+#define FVM_COHERENT_STATES
 #include "fvm_device.cuh"
 #include "fvm_fused.h"
 
@@ -81,7 +82,7 @@ __device__ __forceinline__ int vload(const int *p) { return *reinterpret_cast<co
 // involved-cell lists are built before the launch; never every cell is
 // involved (such steps take the stage kernels).
 template <typename R>
-__global__ void __launch_bounds__(128, FVM_FLUX_MINB(R)) k_rung_step(FusedStep a) {
+__global__ void __launch_bounds__(128, FVM_FLUX_MINB) k_rung_step(FusedStep a) {
   const Params &P = a.P;
   const Dev &d = a.d;
   Sched *S = d.S;

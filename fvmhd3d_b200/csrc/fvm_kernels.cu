@@ -957,7 +957,7 @@ static int enq_corr_flux(fvm_ctx *c) {
   } else if (c->use_flist) {
     CORR_FLUX(LM_EXACT, sgrid(c, c->nf, c->tune.bs_face));
   } else {  // a global step: the instantiation with more resident blocks
-    CORR_FLUX(LM_EXACT, sgrid(c, c->nf, c->tune.bs_face), FVM_GLOBAL_FLUX_MINB(R));
+    CORR_FLUX(LM_EXACT, sgrid(c, c->nf, c->tune.bs_face), FVM_GLOBAL_CORR_MINB(R));
   }
 #undef CORR_FLUX
   LAUNCH_CHECK();
@@ -1119,7 +1119,7 @@ static int enq_update0(fvm_ctx *c) {
   } else if (c->use_flist) {
     PRED_FLUX(LM_EXACT, sgrid(c, c->nf, c->tune.bs_face));
   } else {  // a global step: the instantiation with more resident blocks
-    PRED_FLUX(LM_EXACT, sgrid(c, c->nf, c->tune.bs_face), FVM_GLOBAL_FLUX_MINB(R));
+    PRED_FLUX(LM_EXACT, sgrid(c, c->nf, c->tune.bs_face), FVM_GLOBAL_PRED_MINB(R));
   }
 #undef PRED_FLUX
   LAUNCH_CHECK();

@@ -223,6 +223,17 @@ __device__ __forceinline__ void riemann_hlld(T gamma, T *flux, T Bx, T w, T dens
   flux[WBX] = -w * Bx;
 }
 
+// The normal field of a face state, rounded as the reference's operations are
+// (no contraction) in FP64: the interface psi is a multiple of the difference
+// of the two sides' normal fields, whose round-off is that of the fields
+// themselves, so how it rounds is what the oracle comparison of psi sees.
+__device__ __forceinline__ double dot3_rn(double ax, double ay, double az, double x, double y, double z) {
+  return __dadd_rn(__dadd_rn(__dmul_rn(ax, x), __dmul_rn(ay, y)), __dmul_rn(az, z));
+}
+__device__ __forceinline__ float dot3_rn(float ax, float ay, float az, float x, float y, float z) {
+  return ax * x + ay * y + az * z;
+}
+
 // ---- rotated-frame face flux (MPI/compute_update.cpp:973-1095) -----------
 // Wi/Wj primitive face states, normal the unit normal i->j, wij the face
 // velocity.  Returns the 10 lab-frame fluxes, psi_ij and Bn_ij.
@@ -260,7 +271,7 @@ __device__ __forceinline__ bool compute_flux_with(const Params &P, const T *wij,
   const T velx_L = Axx * Wi[VELX] + Axy * Wi[VELY] + Axz * Wi[VELZ];
   const T vely_L = Ayx * Wi[VELX] + Ayy * Wi[VELY];
   const T velz_L = Azx * Wi[VELX] + Azy * Wi[VELY] + Azz * Wi[VELZ];
-  const T Bx_L = Axx * Wi[BX] + Axy * Wi[BY] + Axz * Wi[BZ];
+  const T Bx_L = dot3_rn(Axx, Axy, Axz, Wi[BX], Wi[BY], Wi[BZ]);
   const T By_L = Ayx * Wi[BX] + Ayy * Wi[BY];
   const T Bz_L = Azx * Wi[BX] + Azy * Wi[BY] + Azz * Wi[BZ];
   const T psiL = Wi[PSI], entrL = Wi[ENTR];
@@ -268,7 +279,7 @@ __device__ __forceinline__ bool compute_flux_with(const Params &P, const T *wij,
   T velx_R = Axx * Wj[VELX] + Axy * Wj[VELY] + Axz * Wj[VELZ];
   const T vely_R = Ayx * Wj[VELX] + Ayy * Wj[VELY];
   const T velz_R = Azx * Wj[VELX] + Azy * Wj[VELY] + Azz * Wj[VELZ];
-  const T Bx_R = Axx * Wj[BX] + Axy * Wj[BY] + Axz * Wj[BZ];
+  const T Bx_R = dot3_rn(Axx, Axy, Axz, Wj[BX], Wj[BY], Wj[BZ]);
   const T By_R = Ayx * Wj[BX] + Ayy * Wj[BY];
   const T Bz_R = Azx * Wj[BX] + Azy * Wj[BY] + Azz * Wj[BZ];
   const T psiR = Wj[PSI], entrR = Wj[ENTR];
