@@ -32,6 +32,10 @@ constexpr int kLimGroup = 4;
 // above the longest stage of a step this kernel runs (the sequential
 // adjust_timesteps sweep over at most its involved cells).
 constexpr long long kBarrierPolls = 1ll << 24;
+#ifndef FVM_FUSED_WIDE
+#define FVM_FUSED_WIDE 2048
+#endif
+constexpr int kWide = FVM_FUSED_WIDE;
 
 __device__ __forceinline__ unsigned load_acquire(const unsigned *p) {
   unsigned v;
@@ -40,39 +44,40 @@ __device__ __forceinline__ unsigned load_acquire(const unsigned *p) {
 }
 
 // Grid-wide barrier over the nblocks working blocks of the launch (the
-// first nblocks; the others have returned).  bar[0] counts arrivals
-// (zero between barriers), bar[1] is the generation, which carries over from
-// launch to launch: each block reads it on entry, and no barrier can complete
-// before every block has arrived, so every block starts from the same value.
-// Thread 0 of each block arrives after a release fence and waits, with
-// bounded polls, for the generation its barrier completes; the last arrival
-// resets the count and publishes the generation.  Returns false on every
-// thread of the block if the wait gave up (err bit 1 set).
-__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned &gen, int *err, unsigned nblocks) {
+// first nblocks; the others have returned).  bar[0] counts arrivals, zero at
+// the start of the launch: thread 0 of each block arrives after a release
+// fence and waits, with bounded polls, until the count covers every block's
+// passage of this barrier (`passed` of them before it).  One atomic and the
+// polls are all a barrier costs; the counters are cleared at the end of the
+// launch (grid_done).  Returns false on every thread of the block if the wait
+// gave up (err bit 1 set).
+__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned &passed, int *err, unsigned nblocks) {
   __syncthreads();
+  passed++;
   int ok = 1;
   if (threadIdx.x == 0) {
-    const unsigned target = gen + 1;
+    const unsigned target = passed * nblocks;
     __threadfence();
-    if (atomicAdd(&bar[0], 1u) == nblocks - 1) {
-      atomicExch(&bar[0], 0u);
-      __threadfence();
-      atomicExch(&bar[1], target);
-    } else {
-      long long it = 0;
-      while (load_acquire(&bar[1]) != target) {
-        if (++it > kBarrierPolls) {
-          atomicOr(err, 1);
-          ok = 0;
-          break;
-        }
-        if (it > 4096) __nanosleep(64);  // short waits spin; long ones back off
+    atomicAdd(&bar[0], 1u);
+    long long it = 0;
+    while (load_acquire(&bar[0]) < target) {
+      if (++it > kBarrierPolls) {
+        atomicOr(err, 1);
+        ok = 0;
+        break;
       }
+      if (it > 4096) __nanosleep(64);  // short waits spin; long ones back off
     }
     __threadfence();
   }
-  gen++;
   return __syncthreads_and(ok) != 0;
+}
+// After a block's last barrier: the last block of all clears the counters.
+__device__ __forceinline__ void grid_done(unsigned *bar, unsigned nblocks) {
+  if (threadIdx.x == 0 && atomicAdd(&bar[1], 1u) == nblocks - 1) {
+    bar[0] = 0u;
+    bar[1] = 0u;
+  }
 }
 
 __device__ __forceinline__ int vload(const int *p) { return *reinterpret_cast<const volatile int *>(p); }
@@ -87,19 +92,22 @@ __global__ void __launch_bounds__(128, FVM_FLUX_MINB) k_rung_step(FusedStep a) {
   const Dev &d = a.d;
   Sched *S = d.S;
   const int n = a.n, nf = a.nf;
-  // Every block works: the stages of a small step are bound by the latency
-  // of each thread's walk over its cell's faces, so more threads beat
-  // cheaper barriers (one block per 64 involved cells measured 0.20 ms per
-  // 200-cell step against 0.15 ms with the whole grid).
-  const unsigned nwork = gridDim.x;
+  // The stages of a small step are bound by the latency of each thread's walk
+  // over its cell's faces, so more threads beat cheaper barriers: one block
+  // per SM works however few the cells (one block per 64 involved cells
+  // measured 0.20 ms per 200-cell step against 0.15 ms).  From kWide involved
+  // cells on the threads' rounds over the cells bound it, and every block of
+  // the launch works; the others return at once.
+  const unsigned nwork = S->ninv >= kWide ? gridDim.x : min(gridDim.x, (unsigned)a.narrow);
+  if (blockIdx.x >= nwork) return;
   const int gt = blockIdx.x * blockDim.x + threadIdx.x, gn = (int)nwork * blockDim.x;
   // lane groups of the cell passes that split a cell's faces (same sums, in
   // the same order, as one thread per cell)
   const int gl = threadIdx.x & (kCellGroup - 1);
   const unsigned gmask = ((1u << kCellGroup) - 1u) << ((threadIdx.x & 31) & ~(kCellGroup - 1));
-  unsigned gen = load_acquire(&a.gbar[1]);
+  unsigned passed = 0;
 #define FVM_GRID_SYNC() \
-  if (!grid_barrier(a.gbar, gen, a.gerr, nwork)) return
+  if (!grid_barrier(a.gbar, passed, a.gerr, nwork)) return
   // the work arrays of adjust_timesteps start cleared for the step's
   // involved cells (the separate-kernel step clears them for every cell).
   // Every entry this step writes or reads is an involved cell's: marks and
@@ -223,6 +231,7 @@ __global__ void __launch_bounds__(128, FVM_FLUX_MINB) k_rung_step(FusedStep a) {
                                                            (R *)d.mnmx, d.mz, (const R *)d.lrw, (const R *)d.lrd, d.csum,
                                                            d.clist, d.bnb, gt, gn);
   if (gt == 0) S->fused_steps += 1;
+  grid_done(a.gbar, nwork);
 #undef FVM_GRID_SYNC
 }
 

@@ -12,19 +12,19 @@ struct FusedStep {
   Dev d;
   LearnBuf lb;
   int n, nf;
-  unsigned *gbar;  // grid barrier: arrivals (zero between launches), generation
+  int narrow;      // blocks that work in a step with few involved cells
+  unsigned *gbar;  // grid barrier: arrivals and finished blocks (zero between launches)
   int *gerr;       // bit 1: a grid barrier wait gave up
 };
 
 // Enqueues one persistent launch of the partial step on `st`: every stage
 // from the slope limiter to the reconstruction over the step's involved
 // cells and active faces, with grid-wide barriers between the stages.  grid:
-// fused_step_blocks_per_sm times the SM count.  Returns the CUDA error of the
-// launch.
+// at most fused_step_blocks_per_sm times the SM count.  Returns the CUDA error
+// of the launch.
 cudaError_t fused_step_enqueue(const FusedStep &a, bool fp32, int grid, cudaStream_t st);
 
-// Blocks of the persistent kernel resident per SM (its grid is this times
-// the SM count).
+// Blocks of the persistent kernel resident per SM.
 int fused_step_blocks_per_sm(bool fp32);
 
 }  // namespace fvm

@@ -1181,7 +1181,7 @@ static int enq_stages(fvm_ctx *c, int shared) {
 // limit): a step it runs involves few cells, and fewer blocks make each grid
 // barrier cheaper.
 #ifndef FVM_FUSED_BPSM
-#define FVM_FUSED_BPSM 1
+#define FVM_FUSED_BPSM 4
 #endif
 
 // Sets the branch of a captured partial step: the persistent rung kernel
@@ -1218,7 +1218,7 @@ static int enq_fused_or_stages(fvm_ctx *c) {
   // if: the persistent kernel (one plain kernel node), captured from the
   // auxiliary stream
   CK(cudaStreamBeginCaptureToGraph(c->aux, body_fused, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-  const FusedStep a = {c->P, c->d, c->lb, c->n, c->nf, c->gbar, c->gerr};
+  const FusedStep a = {c->P, c->d, c->lb, c->n, c->nf, c->sms, c->gbar, c->gerr};
   const cudaError_t le = fused_step_enqueue(a, c->fp32, std::min(c->fused_bpsm, FVM_FUSED_BPSM) * c->sms, c->aux);
   cudaGraph_t done = nullptr;
   const cudaError_t ee = cudaStreamEndCapture(c->aux, &done);
@@ -1261,7 +1261,7 @@ static int enq_step(fvm_ctx *c, int shared) {
     CK(cudaStreamSynchronize(c->st));
     if (ninv <= c->fused_max && ninv < c->n) {
       kt_begin(c, KT_FUSED);
-      const FusedStep a = {c->P, c->d, c->lb, c->n, c->nf, c->gbar, c->gerr};
+      const FusedStep a = {c->P, c->d, c->lb, c->n, c->nf, c->sms, c->gbar, c->gerr};
       CK(fused_step_enqueue(a, c->fp32, std::min(c->fused_bpsm, FVM_FUSED_BPSM) * c->sms, c->st));
       c->launches += 1;
       kt_end(c, KT_FUSED);
