@@ -601,6 +601,15 @@ __global__ void k_link_recon(int n, Params P, const int *FVM_RESTRICT off, const
   store_n<double, 6>(csum + 6 * (size_t)c, sum);
 }
 
+// Lanes per cell of the stage kernels in partial steps of few cells: the walk
+// over a cell's faces is then 1 / STEP_LANES as deep, which is what a small
+// step waits for (the same sums in the same order, so the same bits; steps of
+// one to some hundred active cells 25 to 40 us shorter of 125 to 200).  Every
+// lane repeats its cell's sums, so with many cells one thread each is faster:
+// the corrector cells of a step with 24,389 take 25 us, with lanes 45.
+constexpr int STEP_LANES = 8, FEW_CELLS = 4096;
+__device__ __forceinline__ bool few_cells(const int *clist, int cnt) { return clist && cnt <= FEW_CELLS; }
+
 // ---- slope_limiter (MPI/compute_reconstruction.cpp:201-602) --------------
 // TPC threads per imported cell, each owning KH of the ten primitives: face
 // pass 1 (min/max of neighbour differences) and face pass 2 (limiter of the
@@ -1043,6 +1052,14 @@ __device__ __forceinline__ void limiter_dev(int n, Params P, const Sched *FVM_RE
   // TPC threads per cell; in partial steps a fixed grid strides over clist
   const long long cnt = (long long)TPC * (clist ? S->ninv : n);
   const bool lst = clist && S->ninv != n;  // every cell involved: the list is the identity
+  constexpr int LL = 4;  // lanes per cell and primitive pair
+  if (few_cells(clist, S->ninv) && lst && !reuse) {
+    const unsigned gmask = ((1u << LL) - 1u) << ((threadIdx.x & 31) & ~(LL - 1));
+    for (int t = gt0_ / LL; t < (int)cnt; t += gnt_ / LL)
+      limiter_group<R, KH, LL>(clist[t / TPC], (t % TPC) * KH, gt0_ & (LL - 1), gmask, t_global, off, lfj, fflag, act,
+                               tlast, Wrec, tau, fst, lld);
+    return;
+  }
   for (long long t = (long long)gt0_; t < cnt;
        t += (long long)gnt_) {
     const int u = (int)(t / TPC);
@@ -1525,7 +1542,7 @@ __device__ __forceinline__ void pvel_body(int i, const Params &P, const unsigned
 
 // One thread per cell; in partial steps a fixed grid strides over the
 // involved-cell list (clist, count ninv) instead of every cell.
-template <typename R>
+template <typename R, bool LIST>
 __device__ __forceinline__ void corr_cell_dev(int n, Params P, const Sched *FVM_RESTRICT S,
     const int *FVM_RESTRICT off, const int2 *FVM_RESTRICT lfj, const int2 *FVM_RESTRICT s12,
     const double *FVM_RESTRICT cvol, const unsigned char *FVM_RESTRICT act, const int *FVM_RESTRICT bnd,
@@ -1539,24 +1556,37 @@ __device__ __forceinline__ void corr_cell_dev(int n, Params P, const Sched *FVM_
   const double t_global = S->t_global;
   const int cnt = clist ? S->ninv : n;
   const bool lst = clist && cnt != n;  // every cell involved: the list is the identity
+  // When a whole step runs (Wst not null), compute_pvel and the primitives of
+  // distribute_fluid_update_data of the same cell: its own updated state,
+  // which no later stage changes, in one conversion.
+  auto whole = [&](int c) {
+    const unsigned char ac = act[c];
+    if (!Wst || !(ac & (A_ACTIVE | A_LNGB))) return;
+    double u[NF], W[NF];
+    load_n<double, NF>(U + 10 * (size_t)c, u);
+    to_primitive(u, volp[c], W);
+    R w[NF];
+#pragma unroll
+    for (int k = 0; k < NF; k++) w[k] = R(W[k]);
+    store_n<R, NF>(Wst + 10 * (size_t)c, w);
+    if (ac & A_ACTIVE) pvel_state(c, P, W, bnd, cvol, ccen, pos, vel);
+  };
+  if (LIST && few_cells(clist, cnt)) {
+    const int gl = gt0_ & (STEP_LANES - 1);
+    const unsigned gmask = ((1u << STEP_LANES) - 1u) << ((threadIdx.x & 31) & ~(STEP_LANES - 1));
+    for (int t = gt0_ / STEP_LANES; t < cnt; t += gnt_ / STEP_LANES) {
+      const int c = lst ? clist[t] : t;
+      corr_cell_group<R, STEP_LANES>(c, gl, gmask, t_global, P, off, lfj, cvol, act, bnd, pos, tlast, volp, Wrec, tau,
+                                     fcon, fcode, U, dU, stepdU, counters, divb);
+      if (gl == 0) whole(c);
+    }
+    return;
+  }
   for (int t = gt0_; t < cnt; t += gnt_) {
     const int c = lst ? clist[t] : perm[t];
     corr_cell_body<R>(c, t_global, P, off, lfj, cvol, act, bnd, pos, tlast, volp, Wrec, tau, fcon, fcode, U, dU,
                       stepdU, counters, divb);
-    // When a whole step runs (Wst not null), compute_pvel and the primitives
-    // of distribute_fluid_update_data of the same cell: its own updated state,
-    // which no later stage changes, in one conversion.
-    const unsigned char ac = act[c];
-    if (Wst && (ac & (A_ACTIVE | A_LNGB))) {
-      double u[NF], W[NF];
-      load_n<double, NF>(U + 10 * (size_t)c, u);
-      to_primitive(u, volp[c], W);
-      R w[NF];
-#pragma unroll
-      for (int k = 0; k < NF; k++) w[k] = R(W[k]);
-      store_n<R, NF>(Wst + 10 * (size_t)c, w);
-      if (ac & A_ACTIVE) pvel_state(c, P, W, bnd, cvol, ccen, pos, vel);
-    }
+    whole(c);
   }
 }
 template <typename R>
@@ -1570,7 +1600,7 @@ __global__ void __launch_bounds__(128) k_corr_cell(int n, Params P, const Sched 
     unsigned long long *FVM_RESTRICT counters, const int *FVM_RESTRICT perm, float *FVM_RESTRICT divb,
     const int *FVM_RESTRICT clist, const double *FVM_RESTRICT ccen, double *FVM_RESTRICT vel,
     R *FVM_RESTRICT Wst) {
-  corr_cell_dev<R>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, tlast, volp, Wrec, tau, fcon, fcode, U, dU, stepdU, counters, perm, divb, clist, ccen, vel, Wst, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+  corr_cell_dev<R, true>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, tlast, volp, Wrec, tau, fcon, fcode, U, dU, stepdU, counters, perm, divb, clist, ccen, vel, Wst, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 // The same for global steps, with more resident blocks.
 template <typename R>
@@ -1584,7 +1614,7 @@ __global__ void __launch_bounds__(128, FVM_CORR_CELL_MINB(R)) k_corr_cell_g(int 
     unsigned long long *FVM_RESTRICT counters, const int *FVM_RESTRICT perm, float *FVM_RESTRICT divb,
     const int *FVM_RESTRICT clist, const double *FVM_RESTRICT ccen, double *FVM_RESTRICT vel,
     R *FVM_RESTRICT Wst) {
-  corr_cell_dev<R>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, tlast, volp, Wrec, tau, fcon, fcode, U, dU, stepdU, counters, perm, divb, clist, ccen, vel, Wst, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+  corr_cell_dev<R, false>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, tlast, volp, Wrec, tau, fcon, fcode, U, dU, stepdU, counters, perm, divb, clist, ccen, vel, Wst, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 // Every cell, or in partial steps the involved-cell list.
@@ -1717,9 +1747,9 @@ __global__ void k_timestep(int n, Params P, const int *FVM_RESTRICT off, const i
                            Sched *FVM_RESTRICT S, const int *FVM_RESTRICT clist, int *FVM_RESTRICT aflag,
                            unsigned char *FVM_RESTRICT hash, unsigned char *FVM_RESTRICT act0,
                            unsigned char *FVM_RESTRICT work) {
-  // one thread per cell: every lane of a group would repeat the cell's own
-  // terms (a cube root among them), and on a full step that costs more than
-  // the shorter face walk gains (0.26 -> 0.69 ms on the 128^3 blast)
+  // one thread per cell, but in steps of few cells: every lane of a group
+  // repeats the cell's own terms, and on a full step that costs more than the
+  // shorter face walk gains (0.26 -> 0.69 ms on the 128^3 blast)
   const int gt = blockIdx.x * blockDim.x + threadIdx.x, gn = gridDim.x * blockDim.x;
   if (gt < 4) S->iscal[4 + gt] = 0;
   if (gt < 8) aflag[gt] = 0;
@@ -1733,6 +1763,12 @@ __global__ void k_timestep(int n, Params P, const int *FVM_RESTRICT off, const i
       work[i] = 0;
       work[(size_t)n + i] = 0;
     }
+  }
+  if (few_cells(clist, ninv)) {
+    const unsigned gmask = ((1u << STEP_LANES) - 1u) << ((threadIdx.x & 31) & ~(STEP_LANES - 1));
+    timestep_group<STEP_LANES>(P, off, lfj, act, bnd, U, volp, vel, pos, tlast, tend, dtl, &S->dtmin, clist, ninv,
+                               gt & (STEP_LANES - 1), gmask, gt / STEP_LANES, gn / STEP_LANES, n);
+    return;
   }
   timestep_group<1>(P, off, lfj, act, bnd, U, volp, vel, pos, tlast, tend, dtl, &S->dtmin, clist, ninv, 0,
                     0xffffffffu, gt, gn, n);
@@ -2438,7 +2474,7 @@ __device__ __forceinline__ void pred_cell_group(int c, int gl, unsigned gmask, d
 }
 
 // One thread per cell; in partial steps a fixed grid strides over clist.
-template <typename R>
+template <typename R, bool LIST>
 __device__ __forceinline__ void pred_cell_dev(int n, Params P, const Sched *FVM_RESTRICT S,
     const int *FVM_RESTRICT off, const int2 *FVM_RESTRICT lfj, const int2 *FVM_RESTRICT s12,
     const double *FVM_RESTRICT cvol, const unsigned char *FVM_RESTRICT act, const int *FVM_RESTRICT bnd,
@@ -2450,6 +2486,14 @@ __device__ __forceinline__ void pred_cell_dev(int n, Params P, const Sched *FVM_
   const int min_rung = S->min_rung;
   const int cnt = clist ? S->ninv : n;
   const bool lst = clist && cnt != n;  // every cell involved: the list is the identity
+  if (LIST && few_cells(clist, cnt)) {
+    const int gl = gt0_ & (STEP_LANES - 1);
+    const unsigned gmask = ((1u << STEP_LANES) - 1u) << ((threadIdx.x & 31) & ~(STEP_LANES - 1));
+    for (int t = gt0_ / STEP_LANES; t < cnt; t += gnt_ / STEP_LANES)
+      pred_cell_group<R, STEP_LANES>(lst ? clist[t] : t, gl, gmask, t_global, min_rung, P, off, lfj, cvol, act, bnd, pos,
+                                     U, fcon, fcode, rung, tend, Wrec);
+    return;
+  }
   for (int t = gt0_; t < cnt; t += gnt_)
     pred_cell_body<R>(lst ? clist[t] : perm[t], t_global, min_rung, P, off, lfj, cvol, act, bnd, pos, U, fcon,
                       fcode, rung, tend, Wrec);
@@ -2462,7 +2506,7 @@ __global__ void __launch_bounds__(128) k_pred_cell(int n, Params P, const Sched 
     const R *FVM_RESTRICT fcon, const unsigned char *FVM_RESTRICT fcode,
     int *FVM_RESTRICT rung, double *FVM_RESTRICT tend, R *FVM_RESTRICT Wrec, const int *FVM_RESTRICT perm,
     const int *FVM_RESTRICT clist) {
-  pred_cell_dev<R>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, U, fcon, fcode, rung, tend, Wrec, perm, clist, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+  pred_cell_dev<R, true>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, U, fcon, fcode, rung, tend, Wrec, perm, clist, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 // The same for global steps, with more resident blocks.
 template <typename R>
@@ -2473,7 +2517,7 @@ __global__ void __launch_bounds__(128, FVM_PRED_CELL_MINB(R)) k_pred_cell_g(int 
     const R *FVM_RESTRICT fcon, const unsigned char *FVM_RESTRICT fcode,
     int *FVM_RESTRICT rung, double *FVM_RESTRICT tend, R *FVM_RESTRICT Wrec, const int *FVM_RESTRICT perm,
     const int *FVM_RESTRICT clist) {
-  pred_cell_dev<R>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, U, fcon, fcode, rung, tend, Wrec, perm, clist, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+  pred_cell_dev<R, false>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, U, fcon, fcode, rung, tend, Wrec, perm, clist, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 // ---- compute_reconstruction (MPI/compute_reconstruction.cpp:41-198) -------

@@ -290,6 +290,12 @@ static int sgrid(const fvm_ctx *c, long long items, int bs) {
   return (c->use_flist && g > cap) ? cap : g;
 }
 
+// Grid of a cell kernel: one thread per cell, in partial steps at least the
+// lanes of a step of few cells.
+static int cgrid(const fvm_ctx *c, int bs) {
+  return sgrid(c, c->use_flist ? std::max(c->n, STEP_LANES * FEW_CELLS) : c->n, bs);
+}
+
 static void drop_graphs(fvm_ctx *c) {
   for (int k = 0; k < 2; k++)
     if (c->graph[k]) {
@@ -971,12 +977,12 @@ static int enq_corr_cell(fvm_ctx *c, bool whole) {
   Dev &d = c->d;
   kt_begin(c, KT_CORR_CELL);
 #define CORR_CELL(K)                                                                                           \
-  BULK(K<R><<<sgrid(c, c->n, c->tune.bs_cell), c->tune.bs_cell, 0, c->st>>>(                                   \
+  BULK(K<R><<<cgrid(c, c->tune.bs_cell), c->tune.bs_cell, 0, c->st>>>(                                   \
       c->n, c->P, d.S, d.off, d.lfj, d.s12, d.cvol, d.act, d.bnd, d.pos, d.tlast, d.volp, (const R *)d.Wrec,     \
       (const R *)d.tau, (const R *)d.fcon, d.fcode, d.U, d.dU, d.stepdU, d.counters, d.perm, d.divb,            \
       c->use_flist ? d.clist : nullptr, d.ccen, d.vel, whole ? (R *)d.Wst : nullptr))
-  if (c->use_flist || !c->fp32) CORR_CELL(k_corr_cell);
-  else CORR_CELL(k_corr_cell_g);  // an FP32 global step: more resident blocks
+  if (c->use_flist) CORR_CELL(k_corr_cell);
+  else CORR_CELL(k_corr_cell_g);  // a global step: no list, and in FP32 more resident blocks
 #undef CORR_CELL
   LAUNCH_CHECK();
   kt_end(c, KT_CORR_CELL);
@@ -1004,7 +1010,7 @@ static int enq_timesteps(fvm_ctx *c, int shared) {
   const int n = c->n;
   kt_begin(c, KT_TIMESTEP);
   const int *cl = c->use_flist ? d.clist : nullptr;  // partial steps: the involved cells only
-  k_timestep<<<sgrid(c, n, 128), 128, 0, c->st>>>(n, c->P, d.off, d.lfj, d.act, d.bnd, d.U, d.volp, d.vel,
+  k_timestep<<<cgrid(c, 128), 128, 0, c->st>>>(n, c->P, d.off, d.lfj, d.act, d.bnd, d.U, d.volp, d.vel,
                                                   d.pos, d.tlast, d.tend, d.dtl, d.S, cl, d.aflag, d.hash, d.act0,
                                                   shared ? nullptr : d.awork);
   LAUNCH_CHECK();
@@ -1131,11 +1137,11 @@ static int enq_recon(fvm_ctx *c) {
   Dev &d = c->d;
   kt_begin(c, KT_PRED_CELL);
 #define PRED_CELL(K)                                                                                           \
-  BULK(K<R><<<sgrid(c, c->n, c->tune.bs_cell), c->tune.bs_cell, 0, c->st>>>(                                   \
+  BULK(K<R><<<cgrid(c, c->tune.bs_cell), c->tune.bs_cell, 0, c->st>>>(                                   \
       c->n, c->P, d.S, d.off, d.lfj, d.s12, d.cvol, d.act, d.bnd, d.pos, d.U, (const R *)d.fcon2, d.fcode2,      \
       d.rung, d.tend, (R *)d.Wrec, d.perm, c->use_flist ? d.clist : nullptr))
-  if (c->use_flist || !c->fp32) PRED_CELL(k_pred_cell);
-  else PRED_CELL(k_pred_cell_g);  // an FP32 global step: more resident blocks
+  if (c->use_flist) PRED_CELL(k_pred_cell);
+  else PRED_CELL(k_pred_cell_g);  // a global step: no list, and in FP32 more resident blocks
 #undef PRED_CELL
   LAUNCH_CHECK();
   kt_end(c, KT_PRED_CELL);
