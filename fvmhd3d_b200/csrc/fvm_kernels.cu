@@ -165,6 +165,24 @@ struct fvm_ctx {
   // one captured step per mode (shared / individual), replayed by fvm_run
   cudaGraphExec_t graph[2];
   Sched hS;  // host copy of the device scheduler, refreshed after synchronisation
+  // what a synchronisation reads back, in pinned memory (a pageable copy is
+  // staged, and waits, by itself)
+  struct ReadBack {
+    Sched S;
+    int gerr, counts[2];
+    double dtmin;
+  } *rb_host = nullptr;
+  bool hs_ok = false;  // hS is the device's: nothing was enqueued since it was read
+  int eager_steps = 0;  // consecutive eager global steps of this state (fvm_step)
+  // Work space of calls on host arrays (ws_take), kept up to kKeepBytes and
+  // released with the context.
+  void *ws = nullptr;
+  size_t ws_bytes = 0;
+  // Pinned staging of small calls' host arrays (stage_of): one copy each way
+  // instead of one per array.
+  char *stage = nullptr, *stage_more = nullptr;
+  int staged_calls = 0;
+  long long graph_launches[2] = {};  // kernels of the captured steps
   // learned flux network: image of the FP16 weights and bias operands
   unsigned char *mlp_img = nullptr;
   int *mlp_err = nullptr;
@@ -257,6 +275,49 @@ static int dalloc(fvm_ctx *c, T **p, size_t count) {
   return 0;
 }
 
+// Work space of one call, given back by ws_give after the call's last use on
+// the context's stream.  Up to kKeepBytes it is one buffer kept by the context
+// (allocating and trimming it cost a small call more than its work: 0.58 ms of
+// a gradient of 100 pairs); more is allocated for the call, so that a run that
+// holds most of the memory for its mesh does not hold this too.
+constexpr size_t kKeepBytes = 64u << 20;
+static int ws_take(fvm_ctx *c, void **p, size_t bytes) {
+  *p = nullptr;
+  if (bytes > kKeepBytes) {
+    CK(cudaMallocAsync(p, bytes, c->st));
+    return 0;
+  }
+  if (bytes > c->ws_bytes) {
+    if (c->ws) CK(cudaFreeAsync(c->ws, c->st));
+    c->ws = nullptr;
+    c->ws_bytes = 0;
+    CK(cudaMallocAsync(&c->ws, bytes, c->st));
+    c->ws_bytes = bytes;
+  }
+  *p = c->ws;
+  return 0;
+}
+static int ws_give(fvm_ctx *c, void *p) {
+  if (p && p != c->ws) CK(cudaFreeAsync(p, c->st));
+  return 0;
+}
+// Null where the arrays are copied as they are.  Up to kStageBytes the staging
+// is part of the context's one pinned block.  Pinning more takes as long as some
+// thirty calls save by it (2.5 ms; a batch of 3,000 faces 170 -> 95 us), so a
+// context pins kStageMore when it has made kStageAfter calls of that size.
+constexpr size_t kStageBytes = 64u << 10, kStageMore = 1u << 20;
+constexpr int kStageAfter = 32;
+static char *stage_of(fvm_ctx *c, size_t bytes) {
+  if (bytes <= kStageBytes) return c->stage;
+  if (bytes > kStageMore) return nullptr;
+  if (!c->stage_more && ++c->staged_calls == kStageAfter &&
+      cudaMallocHost((void **)&c->stage_more, kStageMore) != cudaSuccess) {
+    cudaGetLastError();
+    c->stage_more = nullptr;
+  }
+  return c->stage_more;
+}
+
 static int dalloc_bytes(fvm_ctx *c, void **p, size_t bytes) {
   if (*p) cudaFree(*p);
   *p = nullptr;
@@ -297,6 +358,7 @@ static int cgrid(const fvm_ctx *c, int bs) {
 }
 
 static void drop_graphs(fvm_ctx *c) {
+  c->eager_steps = 0;
   for (int k = 0; k < 2; k++)
     if (c->graph[k]) {
       cudaGraphExecDestroy(c->graph[k]);
@@ -309,6 +371,34 @@ static void free_all(fvm_ctx *c) {
   for (size_t k = 0; k < sizeof(Dev) / sizeof(void *); k++)
     if (ptrs[k]) cudaFree(ptrs[k]);
   memset(&c->d, 0, sizeof(Dev));
+}
+
+// The reconstruction of the FP32 bulk path to or from a host array of doubles,
+// converted on the device a piece at a time through the work space.
+constexpr long long kConvertPiece = 4 << 20;  // values
+static int convert_out(fvm_ctx *c, double *host, const float *dev, long long count) {
+  double *tmp = nullptr;
+  int rc = ws_take(c, (void **)&tmp, sizeof(double) * (size_t)std::min(count, kConvertPiece));
+  if (rc) return rc;
+  for (long long o = 0; o < count; o += kConvertPiece) {
+    const long long m = std::min(kConvertPiece, count - o);
+    k_convert<float, double><<<nblk(m, 256), 256, 0, c->st>>>(m, dev + o, tmp);
+    LAUNCH_CHECK();
+    CK(cudaMemcpyAsync(host + o, tmp, (size_t)m * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+  }
+  return ws_give(c, tmp);
+}
+static int convert_in(fvm_ctx *c, float *dev, const double *host, long long count) {
+  double *tmp = nullptr;
+  int rc = ws_take(c, (void **)&tmp, sizeof(double) * (size_t)std::min(count, kConvertPiece));
+  if (rc) return rc;
+  for (long long o = 0; o < count; o += kConvertPiece) {
+    const long long m = std::min(kConvertPiece, count - o);
+    CK(cudaMemcpyAsync(tmp, host + o, (size_t)m * sizeof(double), cudaMemcpyHostToDevice, c->st));
+    k_convert<double, float><<<nblk(m, 256), 256, 0, c->st>>>(m, tmp, dev + o);
+    LAUNCH_CHECK();
+  }
+  return ws_give(c, tmp);
 }
 
 extern "C" {
@@ -348,10 +438,12 @@ fvm_ctx *fvm_create(const fvm_params *p, int device) {
   for (int k = 0; k < 2 * KT_COUNT; k++) cudaEventCreate(&c->kev[k]);
   if (cudaStreamCreateWithFlags(&c->aux, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&c->gbar, 2 * sizeof(unsigned)) != cudaSuccess || cudaMalloc(&c->gerr, sizeof(int)) != cudaSuccess ||
-      cudaMemset(c->gerr, 0, sizeof(int)) != cudaSuccess || cudaMemset(c->gbar, 0, 2 * sizeof(unsigned)) != cudaSuccess) {
+      cudaMemset(c->gerr, 0, sizeof(int)) != cudaSuccess || cudaMemset(c->gbar, 0, 2 * sizeof(unsigned)) != cudaSuccess ||
+      cudaMallocHost((void **)&c->stage, kStageBytes + sizeof(*c->rb_host)) != cudaSuccess) {
     fvm_destroy(c);
     return nullptr;
   }
+  c->rb_host = reinterpret_cast<fvm_ctx::ReadBack *>(c->stage + kStageBytes);
   c->fused_bpsm = fused_step_blocks_per_sm(c->fp32);
   return c;
 }
@@ -368,6 +460,9 @@ void fvm_destroy(fvm_ctx *c) {
   for (int k = 0; k < 2 * KT_COUNT; k++) cudaEventDestroy(c->kev[k]);
   if (c->gbar) cudaFree(c->gbar);
   if (c->gerr) cudaFree(c->gerr);
+  if (c->ws) cudaFreeAsync(c->ws, c->st);
+  if (c->stage) cudaFreeHost(c->stage);
+  if (c->stage_more) cudaFreeHost(c->stage_more);
   cudaEventDestroy(c->ev0);
   cudaEventDestroy(c->ev1);
   if (c->aux) cudaStreamDestroy(c->aux);
@@ -565,10 +660,15 @@ int fvm_set_mesh(fvm_ctx *c, int ncell, int nface, const int *s1, const int *s2,
   return 0;
 }
 
-// Synchronise and refresh the host copy of the scheduler.
+// Synchronise and refresh the host copy of the scheduler (and, with the
+// persistent rung kernel on, of its error bits).
 static int read_sched(fvm_ctx *c) {
-  CK(cudaMemcpyAsync(&c->hS, c->d.S, sizeof(Sched), cudaMemcpyDeviceToHost, c->st));
+  c->rb_host->gerr = 0;
+  CK(cudaMemcpyAsync(&c->rb_host->S, c->d.S, sizeof(Sched), cudaMemcpyDeviceToHost, c->st));
+  if (c->fused_max > 0) CK(cudaMemcpyAsync(&c->rb_host->gerr, c->gerr, sizeof(int), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
+  c->hS = c->rb_host->S;
+  c->hs_ok = true;
   c->tsysU = c->hS.tsysU;
   c->t_global = c->hS.t_global;
   c->min_rung = c->hS.min_rung;
@@ -580,6 +680,7 @@ static int read_sched(fvm_ctx *c) {
 // the end of a step (end) k_sched_begin has zeroed it, and the scheduler's
 // counters are closed too.
 static int enqueue_maxrung(fvm_ctx *c, int end) {
+  c->hs_ok = false;
   if (!end) CK(cudaMemsetAsync(&c->d.S->iscal[0], 0, sizeof(int), c->st));
   k_maxrung<<<smin(nblk(c->n, 256), 4 * c->sms), 256, 0, c->st>>>(c->n, c->d.rung, c->d.S, end);
   LAUNCH_CHECK();
@@ -625,12 +726,14 @@ int fvm_init_problem(fvm_ctx *c, const double *W, const double *pos, const int *
   CK(cudaSetDevice(c->device));
   const int n = c->n;
   Dev &d = c->d;
+  c->hs_ok = false;
   double *dW = nullptr;
-  CK(cudaMalloc(&dW, sizeof(double) * 10 * (size_t)n));
+  int rc = ws_take(c, (void **)&dW, sizeof(double) * 10 * (size_t)n);
+  if (rc) return rc;
   cudaError_t e = cudaMemcpyAsync(dW, W, sizeof(double) * 10 * (size_t)n, cudaMemcpyHostToDevice, c->st);
-  if (e != cudaSuccess) { cudaFree(dW); c->err = cudaGetErrorString(e); return FVM_ECUDA; }
-  int rc = enq_positions(c, pos, bnd);
-  if (rc) { cudaFree(dW); return rc; }
+  if (e != cudaSuccess) { ws_give(c, dW); c->err = cudaGetErrorString(e); return FVM_ECUDA; }
+  rc = enq_positions(c, pos, bnd);
+  if (rc) { ws_give(c, dW); return rc; }
   CK(cudaMemsetAsync(d.vel, 0, sizeof(double) * 3 * (size_t)n, c->st));
   CK(cudaMemsetAsync(d.tlast, 0, sizeof(double) * n, c->st));
 
@@ -652,8 +755,8 @@ int fvm_init_problem(fvm_ctx *c, const double *W, const double *pos, const int *
   LAUNCH_CHECK();
   double dtmin = 0.0;
   CK(cudaMemcpyAsync(&dtmin, &d.S->dtmin, sizeof(double), cudaMemcpyDeviceToHost, c->st));
+  if ((rc = ws_give(c, dW))) return rc;
   CK(cudaStreamSynchronize(c->st));
-  cudaFree(dW);
   if (c->reduce && c->reduce(c->reduce_user, &dtmin) != 0) {
     c->err = "fvm_init_problem: the timestep reduction failed";
     return FVM_EINVAL;
@@ -693,11 +796,8 @@ int fvm_get_state(fvm_ctx *c, double *pos, double *vel, double *tlast, double *t
   if (dU) CK(cudaMemcpyAsync(dU, c->d.dU, 14 * n * sizeof(double), cudaMemcpyDeviceToHost, s));
   if (wrec && !c->fp32) CK(cudaMemcpyAsync(wrec, c->d.Wrec, 50 * n * sizeof(double), cudaMemcpyDeviceToHost, s));
   if (wrec && c->fp32) {
-    double *tmp = nullptr;
-    CK(cudaMallocAsync(&tmp, 50 * n * sizeof(double), s));
-    k_convert<float, double><<<nblk(50LL * n, 256), 256, 0, s>>>(50LL * n, (const float *)c->d.Wrec, tmp);
-    CK(cudaMemcpyAsync(wrec, tmp, 50 * n * sizeof(double), cudaMemcpyDeviceToHost, s));
-    CK(cudaFreeAsync(tmp, s));
+    const int rc = convert_out(c, wrec, (const float *)c->d.Wrec, 50LL * (long long)n);
+    if (rc) return rc;
   }
   CK(cudaStreamSynchronize(s));
   return 0;
@@ -723,11 +823,8 @@ int fvm_set_state(fvm_ctx *c, const double *vel, const double *tlast, const doub
   if (dU) CK(cudaMemcpyAsync(c->d.dU, dU, 14 * n * sizeof(double), cudaMemcpyHostToDevice, s));
   if (wrec && !c->fp32) CK(cudaMemcpyAsync(c->d.Wrec, wrec, 50 * n * sizeof(double), cudaMemcpyHostToDevice, s));
   if (wrec && c->fp32) {
-    double *tmp = nullptr;
-    CK(cudaMallocAsync(&tmp, 50 * n * sizeof(double), s));
-    CK(cudaMemcpyAsync(tmp, wrec, 50 * n * sizeof(double), cudaMemcpyHostToDevice, s));
-    k_convert<double, float><<<nblk(50LL * n, 256), 256, 0, s>>>(50LL * n, tmp, (float *)c->d.Wrec);
-    CK(cudaFreeAsync(tmp, s));
+    const int crc = convert_in(c, (float *)c->d.Wrec, wrec, 50LL * (long long)n);
+    if (crc) return crc;
   }
   CK(cudaMemcpyAsync(c->d.volp, c->d.cvol, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
   k_sched_set<<<1, 1, 0, s>>>(c->P, c->d.S, tsys_ticks, 0);
@@ -852,6 +949,7 @@ static int enq_lists_choice(fvm_ctx *c) {
 }
 
 static int enq_begin(fvm_ctx *c) {
+  c->hs_ok = false;
   const int n = c->n;
   Dev &d = c->d;
   kt_begin(c, KT_FLAGS);
@@ -868,7 +966,7 @@ static int enq_begin(fvm_ctx *c) {
     rc = enq_lists_choice(c);
   } else if (inc && cs == cudaStreamCaptureStatusNone) {
     // an eager step makes the same choice on the host
-    int cnt[2] = {0, 0};
+    int *cnt = c->rb_host->counts;
     CK(cudaMemcpyAsync(&cnt[0], &d.S->iscal[1], sizeof(int), cudaMemcpyDeviceToHost, c->st));
     CK(cudaMemcpyAsync(&cnt[1], &d.S->inc[0], sizeof(int), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
@@ -1018,7 +1116,7 @@ static int enq_timesteps(fvm_ctx *c, int shared) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(c->st, &cs));
     if (cs != cudaStreamCaptureStatusNone) { c->err = "the timestep reduction needs eager steps"; return FVM_EINVAL; }
-    double v = 0.0;
+    double &v = c->rb_host->dtmin;
     CK(cudaMemcpyAsync(&v, &d.S->dtmin, sizeof(double), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     if (c->reduce(c->reduce_user, &v) != 0) { c->err = "the timestep reduction failed"; return FVM_EINVAL; }
@@ -1262,9 +1360,9 @@ static int enq_step(fvm_ctx *c, int shared) {
   } else if (fusable && cs == cudaStreamCaptureStatusNone) {
     // an eager step makes the same choice on the host, from the involved-cell
     // count the step's list building left on the device
-    int ninv = 0;
-    CK(cudaMemcpyAsync(&ninv, &c->d.S->ninv, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(c->rb_host->counts, &c->d.S->ninv, sizeof(int), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
+    const int ninv = c->rb_host->counts[0];
     if (ninv <= c->fused_max && ninv < c->n) {
       kt_begin(c, KT_FUSED);
       const FusedStep a = {c->P, c->d, c->lb, c->n, c->nf, c->sms, c->gbar, c->gerr};
@@ -1322,8 +1420,9 @@ int fvm_compute_timesteps(fvm_ctx *c, int shared, double *dt_min_out) {
   int rc = enq_timesteps(c, shared);
   if (rc) return rc;
   if (dt_min_out) {
-    CK(cudaMemcpyAsync(dt_min_out, &c->d.S->dtmin, sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(&c->rb_host->dtmin, &c->d.S->dtmin, sizeof(double), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
+    *dt_min_out = c->rb_host->dtmin;
   }
   return 0;
 }
@@ -1346,24 +1445,37 @@ int fvm_end_step(fvm_ctx *c, int shared) {
 
 // A grid barrier of the persistent rung kernel that gave up (the step's
 // results are then incomplete): reported, and the barrier cleared.
+// (as of the last read_sched)
 static int check_fused_errors(fvm_ctx *c) {
-  if (c->fused_max <= 0) return 0;
-  int gerr = 0;
-  CK(cudaMemcpy(&gerr, c->gerr, sizeof(int), cudaMemcpyDeviceToHost));
-  if (!gerr) return 0;
+  if (!c->rb_host->gerr) return 0;
   cudaMemset(c->gbar, 0, 2 * sizeof(unsigned));
   cudaMemset(c->gerr, 0, sizeof(int));
   c->err = "a grid barrier of the persistent rung kernel timed out";
   return FVM_ECUDA;
 }
 
+// Global steps of one state replay the captured step from the
+// kGraphAfter-th call on, when its capture has paid off: the launches of an
+// eager step take longer than the kernels of a small mesh.  A host that
+// installs a mesh or state for each step never captures.
+constexpr int kGraphAfter = 8;
+static int step_graph(fvm_ctx *c, int shared);
+
 int fvm_step(fvm_ctx *c, int shared) {
   if (!c || !c->have_state) { if (c) c->err = "fvm_step: no state"; return FVM_ENOMESH; }
   if (c->in_step) { c->err = "fvm_step: inside a step"; return FVM_EINVAL; }
   CK(cudaSetDevice(c->device));
+  int rc = 0;
+  const bool replay = shared && !c->prof && !c->reduce && (c->graph[1] || ++c->eager_steps >= kGraphAfter);
+  if (replay && (rc = step_graph(c, shared))) return rc;
+  c->hs_ok = false;
   CK(cudaEventRecord(c->ev0, c->st));
-  int rc = enq_step(c, shared);
-  if (rc) return rc;
+  if (replay) {
+    CK(cudaGraphLaunch(c->graph[1], c->st));
+    c->launches += c->graph_launches[1];
+  } else if ((rc = enq_step(c, shared))) {
+    return rc;
+  }
   CK(cudaEventRecord(c->ev1, c->st));
   if ((rc = read_sched(c))) return rc;
   if ((rc = check_fused_errors(c))) return rc;
@@ -1401,17 +1513,14 @@ int fvm_step_host(fvm_ctx *c, int shared, unsigned long long tsys_ticks, double 
   const size_t n = c->n;
   cudaStream_t st = c->st, cs = c->cpy;
   const size_t wbytes = 50 * n * sizeof(double);
-  double *wtmp = nullptr;  // the FP32 bulk path converts the reconstruction on the device
   // the inputs the first stages read, on the compute stream
   CK(cudaEventRecord(c->ev0, st));
   CK(cudaMemcpyAsync(d.rung, rung, n * sizeof(int), cudaMemcpyHostToDevice, st));
   if (!c->fp32) {
     CK(cudaMemcpyAsync(d.Wrec, wrec, wbytes, cudaMemcpyHostToDevice, st));
-  } else {
-    CK(cudaMallocAsync(&wtmp, wbytes, st));
-    CK(cudaMemcpyAsync(wtmp, wrec, wbytes, cudaMemcpyHostToDevice, st));
-    k_convert<double, float><<<nblk(50LL * n, 256), 256, 0, st>>>(50LL * n, wtmp, (float *)d.Wrec);
-    LAUNCH_CHECK();
+  } else {  // converted on the device
+    const int crc = convert_in(c, (float *)d.Wrec, wrec, 50LL * (long long)n);
+    if (crc) return crc;
   }
   CK(cudaMemcpyAsync(d.tlast, tlast, n * sizeof(double), cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(d.vel, vel, 3 * n * sizeof(double), cudaMemcpyHostToDevice, st));
@@ -1452,11 +1561,8 @@ int fvm_step_host(fvm_ctx *c, int shared, unsigned long long tsys_ticks, double 
   CK(cudaMemcpyAsync(tend, d.tend, n * sizeof(double), cudaMemcpyDeviceToHost, st));
   if (!c->fp32) {
     CK(cudaMemcpyAsync(wrec, d.Wrec, wbytes, cudaMemcpyDeviceToHost, st));
-  } else {
-    k_convert<float, double><<<nblk(50LL * n, 256), 256, 0, st>>>(50LL * n, (const float *)d.Wrec, wtmp);
-    LAUNCH_CHECK();
-    CK(cudaMemcpyAsync(wrec, wtmp, wbytes, cudaMemcpyDeviceToHost, st));
-    CK(cudaFreeAsync(wtmp, st));
+  } else if ((rc = convert_out(c, wrec, (const float *)d.Wrec, 50LL * (long long)n))) {
+    return rc;
   }
   CK(cudaEventRecord(c->ev1, st));
   CK(cudaStreamSynchronize(cs));
@@ -1468,36 +1574,46 @@ int fvm_step_host(fvm_ctx *c, int shared, unsigned long long tsys_ticks, double 
   return c->hS.iscal[1];
 }
 
+// The captured step of the mode, made on first use.  Per-kernel profiling is
+// not recorded in it.
+static int step_graph(fvm_ctx *c, int shared) {
+  const int g = shared ? 1 : 0;
+  if (c->graph[g]) return 0;
+  const bool prof = c->prof;
+  c->prof = false;
+  cudaGraph_t gr = nullptr;
+  const cudaError_t be = cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal);
+  if (be != cudaSuccess) c->prof = prof;
+  CK(be);
+  const long long l0 = c->launches;
+  const int rc = enq_step(c, shared);
+  c->graph_launches[g] = c->launches - l0;
+  cudaError_t e = cudaStreamEndCapture(c->st, &gr);
+  c->prof = prof;
+  if (rc) { if (gr) cudaGraphDestroy(gr); return rc; }
+  if (e != cudaSuccess) { c->err = std::string("graph capture: ") + cudaGetErrorString(e); return FVM_ECUDA; }
+  e = cudaGraphInstantiate(&c->graph[g], gr, 0);
+  cudaGraphDestroy(gr);
+  if (e != cudaSuccess) { c->graph[g] = nullptr; c->err = std::string("graph instantiate: ") + cudaGetErrorString(e); return FVM_ECUDA; }
+  return 0;
+}
+
 // nsteps steps from one captured CUDA graph per mode, no host round trip
-// between steps.  Per-kernel profiling is not recorded in this mode.
+// between steps.
 int fvm_run(fvm_ctx *c, int nsteps, int shared, long long *faces_out) {
   if (!c || !c->have_state) { if (c) c->err = "fvm_run: no state"; return FVM_ENOMESH; }
   if (c->in_step || nsteps < 0) { c->err = "fvm_run: bad call"; return FVM_EINVAL; }
   if (c->reduce) { c->err = "fvm_run: a timestep reduction is installed (replayed steps cannot call the host)"; return FVM_EINVAL; }
   CK(cudaSetDevice(c->device));
-  const int g = shared ? 1 : 0;
-  if (!c->graph[g]) {
-    const bool prof = c->prof;
-    c->prof = false;
-    cudaGraph_t gr = nullptr;
-    CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
-    int rc = enq_step(c, shared);
-    cudaError_t e = cudaStreamEndCapture(c->st, &gr);
-    c->prof = prof;
-    if (rc) { if (gr) cudaGraphDestroy(gr); return rc; }
-    if (e != cudaSuccess) { c->err = std::string("graph capture: ") + cudaGetErrorString(e); return FVM_ECUDA; }
-    e = cudaGraphInstantiate(&c->graph[g], gr, 0);
-    cudaGraphDestroy(gr);
-    if (e != cudaSuccess) { c->graph[g] = nullptr; c->err = std::string("graph instantiate: ") + cudaGetErrorString(e); return FVM_ECUDA; }
-  }
-  CK(cudaMemcpyAsync(&c->hS, c->d.S, sizeof(Sched), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaStreamSynchronize(c->st));
-  const unsigned long long a0 = c->hS.nactive_total, f0 = c->hS.nfaces_total;
-  CK(cudaEventRecord(c->ev0, c->st));
-  for (int k = 0; k < nsteps; k++) CK(cudaGraphLaunch(c->graph[g], c->st));
-  CK(cudaEventRecord(c->ev1, c->st));
-  int rc = read_sched(c);
+  int rc = step_graph(c, shared);
   if (rc) return rc;
+  if (!c->hs_ok && (rc = read_sched(c))) return rc;
+  const unsigned long long a0 = c->hS.nactive_total, f0 = c->hS.nfaces_total;
+  c->hs_ok = false;
+  CK(cudaEventRecord(c->ev0, c->st));
+  for (int k = 0; k < nsteps; k++) CK(cudaGraphLaunch(c->graph[shared ? 1 : 0], c->st));
+  CK(cudaEventRecord(c->ev1, c->st));
+  if ((rc = read_sched(c))) return rc;
   if ((rc = check_fused_errors(c))) return rc;
   cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1);
   c->max_rung = c->hS.iscal[0];
@@ -1757,24 +1873,35 @@ int fvm_compute_flux(fvm_ctx *c, int nface, const double *wij, const double *Wi,
   if (nface == 0) return 0;
   CK(cudaSetDevice(c->device));
   const size_t nf = nface;
-  const size_t bytes = sizeof(double) * nf * (3 + 10 + 10 + 3 + 1 + 1 + 10) + sizeof(int) * nf;
+  // device layout: wij, Wi, Wj, normal, boundary codes (8 bytes of room each),
+  // then psi, Bn, flux; the host's staging holds the same
+  const size_t in = sizeof(double) * nf * 27, out = sizeof(double) * nf * 12;
   char *buf = nullptr;
-  CK(cudaMalloc(&buf, bytes));
-  double *dw = (double *)buf, *da = dw + 3 * nf, *db = da + 10 * nf, *dn = db + 10 * nf, *dp = dn + 3 * nf,
+  int rc = ws_take(c, (void **)&buf, in + out);
+  if (rc) return rc;
+  double *dw = (double *)buf, *da = dw + 3 * nf, *db = da + 10 * nf, *dn = db + 10 * nf, *dp = dw + 27 * nf,
          *dB = dp + nf, *dF = dB + nf;
-  int *dj = (int *)(dF + 10 * nf);
-  cudaMemcpyAsync(dw, wij, sizeof(double) * 3 * nf, cudaMemcpyHostToDevice, c->st);
-  cudaMemcpyAsync(da, Wi, sizeof(double) * 10 * nf, cudaMemcpyHostToDevice, c->st);
-  cudaMemcpyAsync(db, Wj, sizeof(double) * 10 * nf, cudaMemcpyHostToDevice, c->st);
-  cudaMemcpyAsync(dn, normal, sizeof(double) * 3 * nf, cudaMemcpyHostToDevice, c->st);
-  if (jbnd) cudaMemcpyAsync(dj, jbnd, sizeof(int) * nf, cudaMemcpyHostToDevice, c->st);
+  int *dj = (int *)(dn + 3 * nf);
+  struct Part { const void *host; void *dev; size_t bytes; };
+  const Part ins[] = {{wij, dw, 24 * nf}, {Wi, da, 80 * nf}, {Wj, db, 80 * nf}, {normal, dn, 24 * nf},
+                      {jbnd, dj, sizeof(int) * nf}};
+  const Part outs[] = {{psi, dp, 8 * nf}, {Bn, dB, 8 * nf}, {flux, dF, 80 * nf}};
+  char *st = stage_of(c, std::max(in, out));
+  for (const Part &p : ins) {
+    if (!p.host) continue;
+    if (st) memcpy(st + ((char *)p.dev - buf), p.host, p.bytes);
+    else CK(cudaMemcpyAsync(p.dev, p.host, p.bytes, cudaMemcpyHostToDevice, c->st));
+  }
+  if (st) CK(cudaMemcpyAsync(buf, st, in, cudaMemcpyHostToDevice, c->st));
   k_flux_kat<<<nblk(nface, 128), 128, 0, c->st>>>(nface, c->P, dw, da, db, jbnd ? dj : nullptr, dn, dp, dB, dF);
-  cudaMemcpyAsync(psi, dp, sizeof(double) * nf, cudaMemcpyDeviceToHost, c->st);
-  cudaMemcpyAsync(Bn, dB, sizeof(double) * nf, cudaMemcpyDeviceToHost, c->st);
-  cudaMemcpyAsync(flux, dF, sizeof(double) * 10 * nf, cudaMemcpyDeviceToHost, c->st);
-  cudaError_t e = cudaStreamSynchronize(c->st);
-  cudaFree(buf);
-  if (e != cudaSuccess) { c->err = cudaGetErrorString(e); return FVM_ECUDA; }
+  CK(cudaGetLastError());
+  if (st) CK(cudaMemcpyAsync(st, dp, out, cudaMemcpyDeviceToHost, c->st));
+  else
+    for (const Part &p : outs) CK(cudaMemcpyAsync((void *)p.host, p.dev, p.bytes, cudaMemcpyDeviceToHost, c->st));
+  if ((rc = ws_give(c, buf))) return rc;
+  CK(cudaStreamSynchronize(c->st));
+  if (st)
+    for (const Part &p : outs) memcpy((void *)p.host, st + ((char *)p.dev - (char *)dp), p.bytes);
   return 0;
 }
 
@@ -1951,7 +2078,8 @@ static int mlp_work(fvm_ctx *c, MlpWork &w, long long n, int rows, int hist) {
                           pad(mlpt::I_BYTES / 4)};
   size_t nf = 0;
   for (size_t k : sizes) nf += k;
-  CK(cudaMallocAsync(&w.base, nf * sizeof(float), c->st));
+  int rc = ws_take(c, &w.base, nf * sizeof(float));
+  if (rc) return rc;
   float *p = (float *)w.base;
   float **at[] = {&w.X, &w.T, &w.wt, &w.m, &w.v, &w.grad, &w.hist, &w.part, &w.dz};
   for (int k = 0; k < 9; k++) { *at[k] = p; p += sizes[k]; }
@@ -2000,7 +2128,7 @@ int fvm_mlp_grad(fvm_ctx *c, int n, const float *X, const float *T, const float 
   CK(cudaMemcpyAsync(loss, w.hist, sizeof(float), cudaMemcpyDeviceToHost, c->st));
   int herr = 0;
   CK(cudaMemcpyAsync(&herr, c->mlp_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaFreeAsync(w.base, c->st));
+  if ((rc = ws_give(c, w.base))) return rc;
   CK(cudaStreamSynchronize(c->st));
   if (herr & 4) { c->err = "fvm_mlp_grad: tensor-core product wait timed out"; return FVM_ECUDA; }
   return 0;
@@ -2034,7 +2162,7 @@ int fvm_mlp_train(fvm_ctx *c, long long n, const float *X, const float *T, const
     CK(cudaMemcpyAsync(loss_out, w.hist, (size_t)steps * sizeof(float), cudaMemcpyDeviceToHost, c->st));
   int herr = 0;
   CK(cudaMemcpyAsync(&herr, c->mlp_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaFreeAsync(w.base, c->st));
+  if ((rc = ws_give(c, w.base))) return rc;
   CK(cudaStreamSynchronize(c->st));
   if (herr & 4) { c->err = "fvm_mlp_train: tensor-core product wait timed out"; return FVM_ECUDA; }
   return 0;
@@ -2049,24 +2177,24 @@ int fvm_mlp_eval_counted(fvm_ctx *c, int nmax, int n, const float *X, float *Y) 
   float *dx = nullptr, *dy = nullptr;
   __half *db = nullptr;
   int *dn = nullptr;
-  CK(cudaMallocAsync(&dx, nx * sizeof(float), c->st));
-  CK(cudaMallocAsync(&db, nx * sizeof(__half), c->st));
-  CK(cudaMallocAsync(&dy, ny * sizeof(float), c->st));
-  CK(cudaMallocAsync(&dn, sizeof(int), c->st));
+  char *buf = nullptr;
+  int rc = ws_take(c, (void **)&buf, nx * sizeof(float) + nx * sizeof(__half) + ny * sizeof(float) + 16);
+  if (rc) return rc;
+  dx = (float *)buf;
+  dy = dx + nx;
+  db = (__half *)(dy + ny);
+  dn = (int *)(db + nx);
   CK(cudaMemcpyAsync(dx, X, nx * sizeof(float), cudaMemcpyHostToDevice, c->st));
   CK(cudaMemcpyAsync(dy, Y, ny * sizeof(float), cudaMemcpyHostToDevice, c->st));
   CK(cudaMemcpyAsync(dn, &n, sizeof(int), cudaMemcpyHostToDevice, c->st));
   mlp::k_f32_to_f16<<<(unsigned)((nx + 255) / 256), 256, 0, c->st>>>((long long)nx, dx, db);
   LAUNCH_CHECK();
-  int rc = mlp_launch_dev(c, nmax, dn, db, dy);
+  rc = mlp_launch_dev(c, nmax, dn, db, dy);
   if (rc) return rc;
   CK(cudaMemcpyAsync(Y, dy, ny * sizeof(float), cudaMemcpyDeviceToHost, c->st));
   int herr = 0;
   CK(cudaMemcpyAsync(&herr, c->mlp_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaFreeAsync(dx, c->st));
-  CK(cudaFreeAsync(db, c->st));
-  CK(cudaFreeAsync(dy, c->st));
-  CK(cudaFreeAsync(dn, c->st));
+  if ((rc = ws_give(c, buf))) return rc;
   CK(cudaStreamSynchronize(c->st));
   if (herr) { c->err = "fvm_mlp_eval_counted: tensor-core pipeline wait timed out"; return FVM_ECUDA; }
   return 0;
@@ -2080,20 +2208,21 @@ int fvm_mlp_eval(fvm_ctx *c, int n, const float *X, float *Y) {
   const size_t nx = (size_t)n * mlp::NIN, ny = (size_t)n * mlp::NOUT;
   float *dx = nullptr, *dy = nullptr;
   __half *db = nullptr;
-  CK(cudaMallocAsync(&dx, nx * sizeof(float), c->st));
-  CK(cudaMallocAsync(&db, nx * sizeof(__half), c->st));
-  CK(cudaMallocAsync(&dy, ny * sizeof(float), c->st));
+  char *buf = nullptr;
+  int rc = ws_take(c, (void **)&buf, nx * sizeof(float) + nx * sizeof(__half) + ny * sizeof(float) + 16);
+  if (rc) return rc;
+  dx = (float *)buf;
+  dy = dx + nx;
+  db = (__half *)(dy + ny);
   CK(cudaMemcpyAsync(dx, X, nx * sizeof(float), cudaMemcpyHostToDevice, c->st));
   mlp::k_f32_to_f16<<<(unsigned)((nx + 255) / 256), 256, 0, c->st>>>((long long)nx, dx, db);
   LAUNCH_CHECK();
-  int rc = mlp_launch(c, n, db, dy);
+  rc = mlp_launch(c, n, db, dy);
   if (rc) return rc;
   CK(cudaMemcpyAsync(Y, dy, ny * sizeof(float), cudaMemcpyDeviceToHost, c->st));
   int herr = 0;
   CK(cudaMemcpyAsync(&herr, c->mlp_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaFreeAsync(dx, c->st));
-  CK(cudaFreeAsync(db, c->st));
-  CK(cudaFreeAsync(dy, c->st));
+  if ((rc = ws_give(c, buf))) return rc;
   CK(cudaStreamSynchronize(c->st));
   if (herr) { c->err = "fvm_mlp_eval: tensor-core pipeline wait timed out"; return FVM_ECUDA; }
   return 0;
