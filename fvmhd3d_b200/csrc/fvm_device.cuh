@@ -131,8 +131,15 @@ using namespace fvm;
 #ifndef FVM_PRED_CELL_MINB_F
 #define FVM_PRED_CELL_MINB_F 5
 #endif
-#define FVM_CORR_CELL_MINB(R) (sizeof(R) == 4 ? FVM_CORR_CELL_MINB_F : 1)
-#define FVM_PRED_CELL_MINB(R) (sizeof(R) == 4 ? FVM_PRED_CELL_MINB_F : 1)
+#ifndef FVM_CELL_MINB_D
+#define FVM_CELL_MINB_D 4
+#endif
+#ifndef FVM_GATHER_UNR
+#define FVM_GATHER_UNR 2
+#endif
+#define FVM_CORR_CELL_MINB(R) (sizeof(R) == 4 ? FVM_CORR_CELL_MINB_F : FVM_CELL_MINB_D)
+#define FVM_PRED_CELL_MINB(R) (sizeof(R) == 4 ? FVM_PRED_CELL_MINB_F : FVM_CELL_MINB_D)
+
 #ifndef FVM_CELL_UNROLL
 #define FVM_CELL_UNROLL 1  // unroll factor of the cell kernels' face loops (1 and 2 time the same within 1%)
 #endif
@@ -1281,7 +1288,7 @@ __device__ __forceinline__ void gather_contrib(int c, int q0, int q1, const int2
   double comp[14];
 #pragma unroll
   for (int k = 0; k < 14; k++) { s[k] = 0.0; comp[k] = 0.0; }
-#pragma unroll 2
+FVM_CELL_LOOP_(FVM_GATHER_UNR)
   for (int q = q0; q < q1; q++) {
     const int2 fj = lfj[q];
     const int f = fj.x;
@@ -1665,7 +1672,10 @@ __device__ double cell_timestep(const Params &P, int i, bool with_faces, const i
   double dti = h / (csi + vrel + 1.0 / FVM_HUGE);
   if (with_faces) {
     const double fac = b ? 0.0 : 1.0;
-    double xmax = 0.0;
+    // the largest of the face's speeds, each a square root: the root (and the
+    // sums with it) never decreases with its argument, so the largest argument
+    // gives the largest speed, with two roots instead of two per face
+    double rmax = 0.0, wmax = 0.0;
     const int q0 = off[i], q1 = off[i + 1];
     for (int q = q0 + gl; q < q1; q += G) {
       const int2 fj = lfj[q];
@@ -1674,11 +1684,14 @@ __device__ double cell_timestep(const Params &P, int i, bool with_faces, const i
       const double w3[3] = {(vj[0] + pv[0]) * 0.5, (vj[1] + pv[1]) * 0.5, (vj[2] + pv[2]) * 0.5};
       const double dw[3] = {vj[0] - pv[0], vj[1] - pv[1], vj[2] - pv[2]};
       const double r[3] = {W[VELX] - w3[0], W[VELY] - w3[1], W[VELZ] - w3[2]};
-      const double rv = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
-      const double dwa = sqrt(dw[0] * dw[0] + dw[1] * dw[1] + dw[2] * dw[2]);
-      xmax = smax(xmax, smax(fac * (csi + rv), 1.0 / FVM_HUGE + dwa));
+      rmax = smax(rmax, r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
+      wmax = smax(wmax, dw[0] * dw[0] + dw[1] * dw[1] + dw[2] * dw[2]);
     }
-    for (int o = G / 2; o > 0; o >>= 1) xmax = smax(xmax, __shfl_xor_sync(gmask, xmax, o, G));
+    for (int o = G / 2; o > 0; o >>= 1) {
+      rmax = smax(rmax, __shfl_xor_sync(gmask, rmax, o, G));
+      wmax = smax(wmax, __shfl_xor_sync(gmask, wmax, o, G));
+    }
+    const double xmax = smax(smax(0.0, fac * (csi + sqrt(rmax))), 1.0 / FVM_HUGE + sqrt(wmax));
     if (q1 > q0) dti = smin(dti, h / xmax);
   }
   return dti * P.courant;
