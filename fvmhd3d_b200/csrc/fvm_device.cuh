@@ -2675,9 +2675,6 @@ __global__ void __launch_bounds__(128, MINB) k_recon(int n, Params P, const Sche
   recon_dev<R, KH, MINB>(n, P, S, off, lfj, cvol, act, bnd, Wst, rung, Wrec, perm, mnmx, mz, lrw, lrd, csum, clist, bnb, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
-// Per link (a cell's entry in its face list, i.e. one side of a face), in the
-// order the cell walks its faces: the face id and the neighbour j, stored as
-// ~j when the cell is s2.  The mesh is fixed while it is installed.
 // Cells with a boundary neighbour, whose reconstruction is zero (the
 // reference's face loop stops at such a neighbour,
 // MPI/compute_reconstruction.cpp:103-106,121); boundary codes are fixed
@@ -2692,17 +2689,6 @@ __global__ void k_bnd_neighbours(int n, const int *FVM_RESTRICT off, const int2 
     if (bnd[fj.y >= 0 ? fj.y : ~fj.y] != NO_BOUNDARY) b = 1;
   }
   bnb[c] = b;
-}
-
-__global__ void k_link_tables(int n, const int *FVM_RESTRICT off, const int *FVM_RESTRICT lnk,
-                              const int2 *FVM_RESTRICT s12, int2 *FVM_RESTRICT lfj) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n) return;
-  for (int q = off[c]; q < off[c + 1]; q++) {
-    const int f = lnk[q];
-    const int2 e = s12[f];
-    lfj[q] = make_int2(f, e.x == c ? e.y : ~e.x);
-  }
 }
 
 __global__ void k_shared_sync(int n, Params P, const Sched *FVM_RESTRICT S, const unsigned char *FVM_RESTRICT act,
