@@ -79,6 +79,7 @@ struct Dev {
   // per-step work
   unsigned char *act0, *act, *hash, *fcode, *fcode2, *fflag;
   void *tau, *fcon, *fcon2, *Wst, *fst;  // bulk type
+  double *sums;  // per cell: its summed face contributions (14), of meshes of at least SUM_CELLS cells in FP64
   double *dtl, *stepdU;
   Sched *S;
   unsigned long long *counters;
@@ -134,6 +135,14 @@ using namespace fvm;
 #ifndef FVM_CELL_MINB_D
 #define FVM_CELL_MINB_D 4
 #endif
+// FP64 global steps of at least SUM_CELLS cells sum the face contributions in
+// a pass of their own (k_cell_sums); the cell passes behind it then ask for 5
+// blocks per SM (corrector and predictor cells at 128^3, with the sums: 880
+// and 751 us at 4 blocks, 860 and 741 at 5, 884 and 758 at 6).
+#ifndef FVM_SUMS_MINB
+#define FVM_SUMS_MINB 5
+#endif
+constexpr int SUM_CELLS = 16384, SUM_BLOCK = 224;  // SUM_BLOCK: seven threads for each of 32 cells
 #ifndef FVM_GATHER_UNR
 #define FVM_GATHER_UNR 2
 #endif
@@ -1317,6 +1326,43 @@ FVM_CELL_LOOP_(FVM_GATHER_UNR)
   }
 }
 
+// The sums of gather_contrib of every cell as a pass of their own, in rows of
+// 14, its bits: seven threads per cell, two of the sums each, so that a warp
+// reads a face's record as seven adjacent 16-byte loads.  Both forms wait for
+// loads from L2; one thread per cell loads a record by seven instructions of
+// 32 scattered sectors and needs ~120 registers with the update behind it (16
+// warps per SM), this pass needs few and fills the SM.  Whole cell passes at
+// FP64, one thread per cell -> sums and cells apart: 128^3 corrector 1030 ->
+// 860 us, predictor 896 -> 741; 64^3 160 -> 135 and 143 -> 115.  Steps of
+// 12^3 to 20^3 take the same time either way (75.3 and 75.7 us, 87.5 and
+// 87.5), 32^3 gain 1%, hence SUM_CELLS.  Loops unrolled by 1, 3 or 4 and
+// blocks of 112 or 448 threads measured slower (992, 907, 926, 899, 923 us
+// against 880).  FP32 keeps one thread per cell: its records are half as
+// long, and the compensated sums' state has to travel with them.
+template <bool SKIPJ>
+__global__ void __launch_bounds__(SUM_BLOCK) k_cell_sums(int n, const int *FVM_RESTRICT off,
+    const int2 *FVM_RESTRICT lfj, const double *FVM_RESTRICT fcon, const unsigned char *FVM_RESTRICT fcode,
+    const int *FVM_RESTRICT perm, double *FVM_RESTRICT sums) {
+  const int t = blockIdx.x * (SUM_BLOCK / 7) + threadIdx.x / 7, h = threadIdx.x % 7;
+  if (t >= n) return;
+  const int c = perm[t];
+  const double2 *rec = reinterpret_cast<const double2 *>(fcon) + h;
+  double a = 0.0, b = 0.0;
+  const int q1 = off[c + 1];
+FVM_CELL_LOOP_(FVM_GATHER_UNR)
+  for (int q = off[c]; q < q1; q++) {
+    const int2 fj = lfj[q];
+    const double2 v = __ldg(rec + 7 * (size_t)fj.x);
+    const unsigned char code = fcode[fj.x];
+    const bool is_i = (fj.y >= 0) != ((code & F_SWAP) != 0);
+    const bool use = !(code & F_OFF) && !(!is_i && SKIPJ && (code & F_SKIPJ));
+    const double w = (is_i == (h < NF / 2)) ? -1.0 : 1.0;
+    a = fma(w, use ? v.x : 0.0, a);
+    b = fma(w, use ? v.y : 0.0, b);
+  }
+  reinterpret_cast<double2 *>(sums)[7 * (size_t)c + h] = make_double2(a, b);
+}
+
 // The same sums with G consecutive lanes per cell (G a power of two, gmask
 // the group's lanes, gl this lane's index in it): lane gl loads the records
 // of links q0 + gl, q0 + gl + G, ..., and every lane of the group adds all
@@ -1467,7 +1513,7 @@ __device__ __forceinline__ void corr_cell_finish(int c, unsigned char ac, const 
   store_n<double, NF>(U + 10 * (size_t)c, Un);
 }
 
-template <typename R>
+template <typename R, bool SUMS>
 __device__ __forceinline__ void corr_cell_body(int c, double t_global, const Params &P,
     const int *FVM_RESTRICT off, const int2 *FVM_RESTRICT lfj,
     const double *FVM_RESTRICT cvol, const unsigned char *FVM_RESTRICT act, const int *FVM_RESTRICT bnd,
@@ -1475,11 +1521,12 @@ __device__ __forceinline__ void corr_cell_body(int c, double t_global, const Par
     const R *FVM_RESTRICT Wrec, const R *FVM_RESTRICT tau,
     const R *FVM_RESTRICT fcon, const unsigned char *FVM_RESTRICT fcode,
     double *FVM_RESTRICT U, double *FVM_RESTRICT dU, double *FVM_RESTRICT stepdU,
-    unsigned long long *FVM_RESTRICT counters, float *FVM_RESTRICT divb) {
+    unsigned long long *FVM_RESTRICT counters, float *FVM_RESTRICT divb, const double *FVM_RESTRICT sums) {
   const unsigned char ac = act[c];
   if (!(ac & (A_ACTIVE | A_LNGB))) return;
   double s[14];
-  gather_contrib<R>(c, off[c], off[c + 1], lfj, fcon, fcode, true, s);
+  if (SUMS) load_n<double, 14>(sums + 14 * (size_t)c, s);
+  else gather_contrib<R>(c, off[c], off[c + 1], lfj, fcon, fcode, true, s);
   corr_cell_finish<R>(c, ac, s, t_global, P, cvol, bnd, pos, tlast, volp, Wrec, tau, U, dU, stepdU, counters, divb);
 }
 
@@ -1549,7 +1596,7 @@ __device__ __forceinline__ void pvel_body(int i, const Params &P, const unsigned
 
 // One thread per cell; in partial steps a fixed grid strides over the
 // involved-cell list (clist, count ninv) instead of every cell.
-template <typename R, bool LIST>
+template <typename R, bool LIST, bool SUMS = false>
 __device__ __forceinline__ void corr_cell_dev(int n, Params P, const Sched *FVM_RESTRICT S,
     const int *FVM_RESTRICT off, const int2 *FVM_RESTRICT lfj, const int2 *FVM_RESTRICT s12,
     const double *FVM_RESTRICT cvol, const unsigned char *FVM_RESTRICT act, const int *FVM_RESTRICT bnd,
@@ -1559,7 +1606,7 @@ __device__ __forceinline__ void corr_cell_dev(int n, Params P, const Sched *FVM_
     double *FVM_RESTRICT U, double *FVM_RESTRICT dU, double *FVM_RESTRICT stepdU,
     unsigned long long *FVM_RESTRICT counters, const int *FVM_RESTRICT perm, float *FVM_RESTRICT divb,
     const int *FVM_RESTRICT clist, const double *FVM_RESTRICT ccen, double *FVM_RESTRICT vel,
-    R *FVM_RESTRICT Wst, int gt0_, int gnt_) {
+    R *FVM_RESTRICT Wst, int gt0_, int gnt_, const double *FVM_RESTRICT sums = nullptr) {
   const double t_global = S->t_global;
   const int cnt = clist ? S->ninv : n;
   const bool lst = clist && cnt != n;  // every cell involved: the list is the identity
@@ -1591,8 +1638,8 @@ __device__ __forceinline__ void corr_cell_dev(int n, Params P, const Sched *FVM_
   }
   for (int t = gt0_; t < cnt; t += gnt_) {
     const int c = lst ? clist[t] : perm[t];
-    corr_cell_body<R>(c, t_global, P, off, lfj, cvol, act, bnd, pos, tlast, volp, Wrec, tau, fcon, fcode, U, dU,
-                      stepdU, counters, divb);
+    corr_cell_body<R, SUMS>(c, t_global, P, off, lfj, cvol, act, bnd, pos, tlast, volp, Wrec, tau, fcon, fcode, U,
+                            dU, stepdU, counters, divb, sums);
     whole(c);
   }
 }
@@ -1610,8 +1657,8 @@ __global__ void __launch_bounds__(128) k_corr_cell(int n, Params P, const Sched 
   corr_cell_dev<R, true>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, tlast, volp, Wrec, tau, fcon, fcode, U, dU, stepdU, counters, perm, divb, clist, ccen, vel, Wst, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 // The same for global steps, with more resident blocks.
-template <typename R>
-__global__ void __launch_bounds__(128, FVM_CORR_CELL_MINB(R)) k_corr_cell_g(int n, Params P, const Sched *FVM_RESTRICT S,
+template <typename R, bool SUMS>
+__global__ void __launch_bounds__(128, SUMS ? FVM_SUMS_MINB : FVM_CORR_CELL_MINB(R)) k_corr_cell_g(int n, Params P, const Sched *FVM_RESTRICT S,
     const int *FVM_RESTRICT off, const int2 *FVM_RESTRICT lfj, const int2 *FVM_RESTRICT s12,
     const double *FVM_RESTRICT cvol, const unsigned char *FVM_RESTRICT act, const int *FVM_RESTRICT bnd,
     const double *FVM_RESTRICT pos, const double *FVM_RESTRICT tlast, double *FVM_RESTRICT volp,
@@ -1620,8 +1667,8 @@ __global__ void __launch_bounds__(128, FVM_CORR_CELL_MINB(R)) k_corr_cell_g(int 
     double *FVM_RESTRICT U, double *FVM_RESTRICT dU, double *FVM_RESTRICT stepdU,
     unsigned long long *FVM_RESTRICT counters, const int *FVM_RESTRICT perm, float *FVM_RESTRICT divb,
     const int *FVM_RESTRICT clist, const double *FVM_RESTRICT ccen, double *FVM_RESTRICT vel,
-    R *FVM_RESTRICT Wst) {
-  corr_cell_dev<R, false>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, tlast, volp, Wrec, tau, fcon, fcode, U, dU, stepdU, counters, perm, divb, clist, ccen, vel, Wst, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    R *FVM_RESTRICT Wst, const double *FVM_RESTRICT sums) {
+  corr_cell_dev<R, false, SUMS>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, tlast, volp, Wrec, tau, fcon, fcode, U, dU, stepdU, counters, perm, divb, clist, ccen, vel, Wst, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, sums);
 }
 
 // Every cell, or in partial steps the involved-cell list.
@@ -2458,16 +2505,17 @@ __device__ __forceinline__ void pred_cell_finish(int c, const double *dot, doubl
   tend[c] = t_global + get_dt(P, rf);
 }
 
-template <typename R>
+template <typename R, bool SUMS>
 __device__ __forceinline__ void pred_cell_body(int c, double t_global, int min_rung, const Params &P,
     const int *FVM_RESTRICT off, const int2 *FVM_RESTRICT lfj,
     const double *FVM_RESTRICT cvol, const unsigned char *FVM_RESTRICT act, const int *FVM_RESTRICT bnd,
     const double *FVM_RESTRICT pos, const double *FVM_RESTRICT U,
     const R *FVM_RESTRICT fcon, const unsigned char *FVM_RESTRICT fcode,
-    int *FVM_RESTRICT rung, double *FVM_RESTRICT tend, R *FVM_RESTRICT Wrec) {
+    int *FVM_RESTRICT rung, double *FVM_RESTRICT tend, R *FVM_RESTRICT Wrec, const double *FVM_RESTRICT sums) {
   if (!(act[c] & A_ACTIVE) || bnd[c] != NO_BOUNDARY) return;
   double dot[14];
-  gather_contrib<R>(c, off[c], off[c + 1], lfj, fcon, fcode, false, dot);
+  if (SUMS) load_n<double, 14>(sums + 14 * (size_t)c, dot);
+  else gather_contrib<R>(c, off[c], off[c + 1], lfj, fcon, fcode, false, dot);
   pred_cell_finish<R>(c, dot, t_global, min_rung, P, cvol, pos, U, rung, tend, Wrec);
 }
 
@@ -2487,14 +2535,15 @@ __device__ __forceinline__ void pred_cell_group(int c, int gl, unsigned gmask, d
 }
 
 // One thread per cell; in partial steps a fixed grid strides over clist.
-template <typename R, bool LIST>
+template <typename R, bool LIST, bool SUMS = false>
 __device__ __forceinline__ void pred_cell_dev(int n, Params P, const Sched *FVM_RESTRICT S,
     const int *FVM_RESTRICT off, const int2 *FVM_RESTRICT lfj, const int2 *FVM_RESTRICT s12,
     const double *FVM_RESTRICT cvol, const unsigned char *FVM_RESTRICT act, const int *FVM_RESTRICT bnd,
     const double *FVM_RESTRICT pos, const double *FVM_RESTRICT U,
     const R *FVM_RESTRICT fcon, const unsigned char *FVM_RESTRICT fcode,
     int *FVM_RESTRICT rung, double *FVM_RESTRICT tend, R *FVM_RESTRICT Wrec, const int *FVM_RESTRICT perm,
-    const int *FVM_RESTRICT clist, int gt0_, int gnt_) {
+    const int *FVM_RESTRICT clist, int gt0_, int gnt_,
+    const double *FVM_RESTRICT sums = nullptr) {
   const double t_global = S->t_global;
   const int min_rung = S->min_rung;
   const int cnt = clist ? S->ninv : n;
@@ -2508,8 +2557,8 @@ __device__ __forceinline__ void pred_cell_dev(int n, Params P, const Sched *FVM_
     return;
   }
   for (int t = gt0_; t < cnt; t += gnt_)
-    pred_cell_body<R>(lst ? clist[t] : perm[t], t_global, min_rung, P, off, lfj, cvol, act, bnd, pos, U, fcon,
-                      fcode, rung, tend, Wrec);
+    pred_cell_body<R, SUMS>(lst ? clist[t] : perm[t], t_global, min_rung, P, off, lfj, cvol, act, bnd, pos, U, fcon,
+                            fcode, rung, tend, Wrec, sums);
 }
 template <typename R>
 __global__ void __launch_bounds__(128) k_pred_cell(int n, Params P, const Sched *FVM_RESTRICT S,
@@ -2522,15 +2571,15 @@ __global__ void __launch_bounds__(128) k_pred_cell(int n, Params P, const Sched 
   pred_cell_dev<R, true>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, U, fcon, fcode, rung, tend, Wrec, perm, clist, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 // The same for global steps, with more resident blocks.
-template <typename R>
-__global__ void __launch_bounds__(128, FVM_PRED_CELL_MINB(R)) k_pred_cell_g(int n, Params P, const Sched *FVM_RESTRICT S,
+template <typename R, bool SUMS>
+__global__ void __launch_bounds__(128, SUMS ? FVM_SUMS_MINB : FVM_PRED_CELL_MINB(R)) k_pred_cell_g(int n, Params P, const Sched *FVM_RESTRICT S,
     const int *FVM_RESTRICT off, const int2 *FVM_RESTRICT lfj, const int2 *FVM_RESTRICT s12,
     const double *FVM_RESTRICT cvol, const unsigned char *FVM_RESTRICT act, const int *FVM_RESTRICT bnd,
     const double *FVM_RESTRICT pos, const double *FVM_RESTRICT U,
     const R *FVM_RESTRICT fcon, const unsigned char *FVM_RESTRICT fcode,
     int *FVM_RESTRICT rung, double *FVM_RESTRICT tend, R *FVM_RESTRICT Wrec, const int *FVM_RESTRICT perm,
-    const int *FVM_RESTRICT clist) {
-  pred_cell_dev<R, false>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, U, fcon, fcode, rung, tend, Wrec, perm, clist, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    const int *FVM_RESTRICT clist, const double *FVM_RESTRICT sums) {
+  pred_cell_dev<R, false, SUMS>(n, P, S, off, lfj, s12, cvol, act, bnd, pos, U, fcon, fcode, rung, tend, Wrec, perm, clist, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, sums);
 }
 
 // ---- compute_reconstruction (MPI/compute_reconstruction.cpp:41-198) -------

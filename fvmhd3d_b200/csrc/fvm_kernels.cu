@@ -492,6 +492,9 @@ void fvm_destroy(fvm_ctx *c) {
 
 const char *fvm_last_error(const fvm_ctx *c) { return c ? c->err.c_str() : "null context"; }
 
+// Whether global steps sum the face contributions in a pass of their own.
+static bool cell_sums(const fvm_ctx *c, long long ncell) { return !c->fp32 && ncell >= SUM_CELLS; }
+
 // Device arrays of a mesh with room for ncell cells, nface faces and nl
 // links (cap_* record the room; a mesh that fits reuses them).
 static int alloc_mesh(fvm_ctx *c, long long ncell, long long nface, long long nl) {
@@ -514,6 +517,7 @@ static int alloc_mesh(fvm_ctx *c, long long ncell, long long nface, long long nl
   BULK(rc |= dalloc_bytes(c, &d.lrw, ReconLink<R>::NW * sizeof(R) * (size_t)nl);
        rc |= dalloc_bytes(c, &d.lrd, ReconLink<R>::ND * sizeof(R) * (size_t)nl));
   rc |= dalloc(c, &d.csum, 6 * (size_t)ncell);
+  if (cell_sums(c, ncell)) rc |= dalloc(c, &d.sums, 14 * (size_t)ncell);
   rc |= dalloc_bytes(c, &d.lld, 3 * c->rb * (size_t)nl);
   rc |= dalloc(c, &d.alist, ncell);
   rc |= dalloc(c, &d.pos, 3 * (size_t)ncell); rc |= dalloc(c, &d.vel, 3 * (size_t)ncell);
@@ -1090,13 +1094,21 @@ static int enq_corr_flux(fvm_ctx *c) {
 static int enq_corr_cell(fvm_ctx *c, bool whole) {
   Dev &d = c->d;
   kt_begin(c, KT_CORR_CELL);
-#define CORR_CELL(K)                                                                                           \
-  BULK(K<R><<<cgrid(c, c->tune.bs_cell), c->tune.bs_cell, 0, c->st>>>(                                   \
+#define CORR_CELL(K, ...)                                                                                      \
+  BULK(K<<<cgrid(c, c->tune.bs_cell), c->tune.bs_cell, 0, c->st>>>(                                   \
       c->n, c->P, d.S, d.off, d.lfj, d.s12, d.cvol, d.act, d.bnd, d.pos, d.tlast, d.volp, (const R *)d.Wrec,     \
       (const R *)d.tau, (const R *)d.fcon, d.fcode, d.U, d.dU, d.stepdU, d.counters, d.perm, d.divb,            \
-      c->use_flist ? d.clist : nullptr, d.ccen, d.vel, whole ? (R *)d.Wst : nullptr))
-  if (c->use_flist) CORR_CELL(k_corr_cell);
-  else CORR_CELL(k_corr_cell_g);  // a global step: no list, and in FP32 more resident blocks
+      c->use_flist ? d.clist : nullptr, d.ccen, d.vel, whole ? (R *)d.Wst : nullptr, ##__VA_ARGS__))
+  if (c->use_flist) {
+    CORR_CELL((k_corr_cell<R>));
+  } else if (cell_sums(c, c->n)) {
+    k_cell_sums<true><<<(c->n + SUM_BLOCK / 7 - 1) / (SUM_BLOCK / 7), SUM_BLOCK, 0, c->st>>>(
+        c->n, d.off, d.lfj, (const double *)d.fcon, d.fcode, d.perm, d.sums);
+    LAUNCH_CHECK();
+    CORR_CELL((k_corr_cell_g<R, true>), d.sums);
+  } else {  // a global step: no list, and in FP32 more resident blocks
+    CORR_CELL((k_corr_cell_g<R, false>), nullptr);
+  }
 #undef CORR_CELL
   LAUNCH_CHECK();
   kt_end(c, KT_CORR_CELL);
@@ -1250,12 +1262,20 @@ static int enq_update0(fvm_ctx *c) {
 static int enq_recon(fvm_ctx *c) {
   Dev &d = c->d;
   kt_begin(c, KT_PRED_CELL);
-#define PRED_CELL(K)                                                                                           \
-  BULK(K<R><<<cgrid(c, c->tune.bs_cell), c->tune.bs_cell, 0, c->st>>>(                                   \
+#define PRED_CELL(K, ...)                                                                                      \
+  BULK(K<<<cgrid(c, c->tune.bs_cell), c->tune.bs_cell, 0, c->st>>>(                                   \
       c->n, c->P, d.S, d.off, d.lfj, d.s12, d.cvol, d.act, d.bnd, d.pos, d.U, (const R *)d.fcon2, d.fcode2,      \
-      d.rung, d.tend, (R *)d.Wrec, d.perm, c->use_flist ? d.clist : nullptr))
-  if (c->use_flist) PRED_CELL(k_pred_cell);
-  else PRED_CELL(k_pred_cell_g);  // a global step: no list, and in FP32 more resident blocks
+      d.rung, d.tend, (R *)d.Wrec, d.perm, c->use_flist ? d.clist : nullptr, ##__VA_ARGS__))
+  if (c->use_flist) {
+    PRED_CELL((k_pred_cell<R>));
+  } else if (cell_sums(c, c->n)) {
+    k_cell_sums<false><<<(c->n + SUM_BLOCK / 7 - 1) / (SUM_BLOCK / 7), SUM_BLOCK, 0, c->st>>>(
+        c->n, d.off, d.lfj, (const double *)d.fcon2, d.fcode2, d.perm, d.sums);
+    LAUNCH_CHECK();
+    PRED_CELL((k_pred_cell_g<R, true>), d.sums);
+  } else {  // a global step: no list, and in FP32 more resident blocks
+    PRED_CELL((k_pred_cell_g<R, false>), nullptr);
+  }
 #undef PRED_CELL
   LAUNCH_CHECK();
   kt_end(c, KT_PRED_CELL);
