@@ -123,9 +123,8 @@ using namespace fvm;
 // Resident blocks per SM that the FP32 global-step instantiations of the
 // compute_update and compute_update0 cell passes ask for.  Measured on the
 // 128^3 blast: corrector cells 1.04 -> 0.78 ms and predictor cells 0.77 ->
-// 0.74 ms at 5 (96 registers, a few bytes of spills).  FP64 global steps
-// launch the partial-step kernels (the FP64 instantiations of the global
-// ones are built but not launched).
+// 0.74 ms at 5 (96 registers, a few bytes of spills).  FP64 ones without a pass
+// of sums ask for 4 (1040 us at 128^3; 1051, 1075 and 1123 at 5, 6 and 7).
 #ifndef FVM_CORR_CELL_MINB_F
 #define FVM_CORR_CELL_MINB_F 5
 #endif

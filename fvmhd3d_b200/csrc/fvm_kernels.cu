@@ -181,8 +181,7 @@ struct fvm_ctx {
   // one captured step per mode (shared / individual), replayed by fvm_run
   cudaGraphExec_t graph[2];
   Sched hS;  // host copy of the device scheduler, refreshed after synchronisation
-  // what a synchronisation reads back, in pinned memory (a pageable copy is
-  // staged, and waits, by itself)
+  // what a synchronisation reads back, behind the staging (stage)
   struct ReadBack {
     Sched S;
     int gerr, counts[2];
@@ -194,10 +193,11 @@ struct fvm_ctx {
   // released with the context.
   void *ws = nullptr;
   size_t ws_bytes = 0;
-  // Pinned staging of small calls' host arrays (stage_of): one copy each way
-  // instead of one per array.
+  // Staging of small calls' host arrays (stage_of): one copy each way instead
+  // of one per array.  stage is plain memory until pin_stage pins it.
   char *stage = nullptr, *stage_more = nullptr;
-  int staged_calls = 0;
+  bool stage_pinned = false;
+  int small_calls = 0, staged_calls = 0;
   long long graph_launches[2] = {};  // kernels of the captured steps
   // learned flux network: image of the FP16 weights and bias operands
   unsigned char *mlp_img = nullptr;
@@ -318,20 +318,47 @@ static int ws_give(fvm_ctx *c, void *p) {
   if (p && p != c->ws) CK(cudaFreeAsync(p, c->st));
   return 0;
 }
-// Null where the arrays are copied as they are.  Up to kStageBytes the staging
-// is part of the context's one pinned block.  Pinning more takes as long as some
-// thirty calls save by it (2.5 ms; a batch of 3,000 faces 170 -> 95 us), so a
-// context pins kStageMore when it has made kStageAfter calls of that size.
-constexpr size_t kStageBytes = 64u << 10, kStageMore = 1u << 20;
-constexpr int kStageAfter = 32;
-static char *stage_of(fvm_ctx *c, size_t bytes) {
-  if (bytes <= kStageBytes) return c->stage;
-  if (bytes > kStageMore) return nullptr;
-  if (!c->stage_more && ++c->staged_calls == kStageAfter &&
-      cudaMallocHost((void **)&c->stage_more, kStageMore) != cudaSuccess) {
+// Pinned host memory, or null (the caller goes on without); also while another
+// thread of the process captures a graph.
+static void *pinned(size_t bytes) {
+  void *p = nullptr;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (cudaMallocHost(&p, bytes) != cudaSuccess) {
     cudaGetLastError();
-    c->stage_more = nullptr;
+    p = nullptr;
   }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return p;
+}
+// Pinning takes 2.5 ms whatever the size, as long as some hundred calls save by
+// it (a pageable copy is staged, and waits, by itself): the context's block
+// (kStageBytes of staging and what a synchronisation reads back) is plain
+// memory until kPinAfter calls have used it, so that creating a context does
+// not pay for it.  Called where no copy of the block is in flight.
+constexpr size_t kStageBytes = 64u << 10, kStageMore = 1u << 20;
+constexpr int kPinAfter = 64, kStageAfter = 32;
+static void pin_stage(fvm_ctx *c) {
+  if (c->stage_pinned || c->small_calls >= kPinAfter || ++c->small_calls < kPinAfter) return;
+  char *p = (char *)pinned(kStageBytes + sizeof(*c->rb_host));
+  if (!p) return;
+  memcpy(p + kStageBytes, c->rb_host, sizeof(*c->rb_host));
+  free(c->stage);
+  c->stage = p;
+  c->rb_host = reinterpret_cast<fvm_ctx::ReadBack *>(p + kStageBytes);
+  c->stage_pinned = true;
+}
+// Null where the arrays are copied as they are.  Up to kStageBytes the staging
+// is part of the context's one block; a call of up to kStageMore saves more by
+// pinned staging (a batch of 3,000 faces 170 -> 95 us), so a context pins that
+// much when it has made kStageAfter such calls.
+static char *stage_of(fvm_ctx *c, size_t bytes) {
+  if (bytes <= kStageBytes) {
+    pin_stage(c);
+    return c->stage;
+  }
+  if (bytes > kStageMore) return nullptr;
+  if (!c->stage_more && ++c->staged_calls == kStageAfter) c->stage_more = (char *)pinned(kStageMore);
   return c->stage_more;
 }
 
@@ -456,7 +483,7 @@ fvm_ctx *fvm_create(const fvm_params *p, int device) {
   if (cudaStreamCreateWithFlags(&c->aux, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&c->gbar, 2 * sizeof(unsigned)) != cudaSuccess || cudaMalloc(&c->gerr, sizeof(int)) != cudaSuccess ||
       cudaMemset(c->gerr, 0, sizeof(int)) != cudaSuccess || cudaMemset(c->gbar, 0, 2 * sizeof(unsigned)) != cudaSuccess ||
-      cudaMallocHost((void **)&c->stage, kStageBytes + sizeof(*c->rb_host)) != cudaSuccess) {
+      !(c->stage = (char *)calloc(1, kStageBytes + sizeof(*c->rb_host)))) {
     fvm_destroy(c);
     return nullptr;
   }
@@ -478,7 +505,8 @@ void fvm_destroy(fvm_ctx *c) {
   if (c->gbar) cudaFree(c->gbar);
   if (c->gerr) cudaFree(c->gerr);
   if (c->ws) cudaFreeAsync(c->ws, c->st);
-  if (c->stage) cudaFreeHost(c->stage);
+  if (c->stage_pinned) cudaFreeHost(c->stage);
+  else free(c->stage);
   if (c->stage_more) cudaFreeHost(c->stage_more);
   cudaEventDestroy(c->ev0);
   cudaEventDestroy(c->ev1);
@@ -683,6 +711,7 @@ int fvm_set_mesh(fvm_ctx *c, int ncell, int nface, const int *s1, const int *s2,
 // Synchronise and refresh the host copy of the scheduler (and, with the
 // persistent rung kernel on, of its error bits).
 static int read_sched(fvm_ctx *c) {
+  pin_stage(c);
   c->rb_host->gerr = 0;
   CK(cudaMemcpyAsync(&c->rb_host->S, c->d.S, sizeof(Sched), cudaMemcpyDeviceToHost, c->st));
   if (c->fused_max > 0) CK(cudaMemcpyAsync(&c->rb_host->gerr, c->gerr, sizeof(int), cudaMemcpyDeviceToHost, c->st));
@@ -1945,12 +1974,11 @@ int fvm_compute_flux(fvm_ctx *c, int nface, const double *wij, const double *Wi,
 
 // ==================== fvm_compute_flux_static (no allocation) ====================
 //
-// fvm_compute_flux stages its face batch in a device buffer it cudaMallocs and
-// cudaFrees on every call.  Some callers cannot do that while they run: a host
+// fvm_compute_flux stages its face batch in device work space that its context
+// allocates when a batch needs more than it keeps.  Some callers cannot do that while they run: a host
 // integrator that solves boundary or sub-grid face batches between steps of a
-// GPU pipeline whose other streams stay busy (cudaFree waits for the whole
-// device, stalling them), and a run that holds most of HBM for its mesh, where
-// a per-call cudaMalloc can fail half way through.  fvm_compute_flux_static
+// GPU pipeline whose other streams stay busy, and a run that holds most of HBM
+// for its mesh, where an allocation can fail half way through.  fvm_compute_flux_static
 // runs the same kernel (k_flux_kat) on the same inputs with its staging in the
 // file-scope array below instead, and calls no allocating routine.
 //

@@ -232,9 +232,8 @@ int fvm_compute_flux(fvm_ctx *c, int nface, const double *wij, const double *Wi,
 /* No counterpart in the reference.  fvm_compute_flux without device
  * allocation, for callers that must not allocate while they run: a host
  * integrator solving boundary or sub-grid face batches between steps while
- * other streams keep the GPU busy (fvm_compute_flux's per-call cudaFree waits
- * for the whole device), or a run holding most of HBM for its mesh, where a
- * per-call cudaMalloc can fail mid-run.  Same arguments and results as
+ * other streams keep the GPU busy, or a run holding most of HBM for its mesh,
+ * where fvm_compute_flux's work space can fail to grow mid-run.  Same arguments and results as
  * fvm_compute_flux; the batch is staged in one fixed device array of
  * FVM_FLUX_STATIC_MAX_FACES faces (about 5 MB) that every call on a device
  * shares.  nface above the capacity returns FVM_ERANGE and does nothing.

@@ -48,3 +48,23 @@ def test_steps_after_the_first_eager_ones(precision):
     a, b = eager.get_state(), later.get_state()
     for k in a:
         assert np.array_equal(a[k], b[k]), k
+
+
+def test_calls_across_the_pinning_of_the_small_staging():
+    """The staging of small calls becomes pinned memory after 64 of them."""
+    m = F.build_periodic(F.jittered_lattice(5, 0.1, seed=5), 1.0)
+    W = F.problems.blast(m.pos)
+    s, plain = F.System(), F.System()
+    for x in (s, plain):
+        x.set_mesh(m)
+        x.init_problem(W)
+    args = face_batch(40, seed=6)
+    want = F.System().compute_flux(*args)
+    for k in range(50):
+        assert s.step(shared=True) == plain.step(shared=True)
+        assert s.clock() == plain.clock()
+        for a, b in zip(s.compute_flux(*args), want):
+            assert np.array_equal(a, b, equal_nan=True)
+    a, b = s.get_state(), plain.get_state()
+    for k in a:
+        assert np.array_equal(a[k], b[k]), k
