@@ -67,25 +67,26 @@ def kernel_bytes(name, N, F, prec_bytes=8):
 
 
 # DRAM bytes (read + write) per launch measured by ncu on the 64^3 blast
-# (262144 cells, 2085347 faces; profiles/cell_and_face_kernels_blast64_*_full.md),
-# per face; a launch on another mesh of the same kind moves these bytes times
+# (262144 cells, 2085347 faces; profiles/global_step_kernels_blast64_fp64.md and
+# cell_and_face_kernels_blast64_fp32_full.md; FP64 cell passes with their pass of
+# sums), per face; a launch on another mesh of the same kind moves these bytes times
 # its face count.
 NCU_FACES_64 = 2085347
 NCU_TRAFFIC_64 = {
-    ("limiter", 8): 293.388800e6 + 305.387264e6, ("limiter", 4): 168.422656e6 + 129.603584e6,
-    ("corr_flux", 8): 495.818752e6 + 205.004032e6, ("corr_flux", 4): 328.471296e6 + 95.712000e6,
-    ("corr_cell", 8): 460.649728e6 + 42.046464e6, ("corr_cell", 4): 275.880960e6 + 34.968064e6,
-    ("pred_flux", 8): 181.350912e6 + 183.134720e6, ("pred_flux", 4): 170.220032e6 + 84.814848e6,
-    ("pred_cell", 8): 353.519104e6 + 24.941824e6, ("pred_cell", 4): 192.598272e6 + 16.507392e6,
-    ("recon", 8): 416.417024e6 + 127.086336e6, ("recon", 4): 243.891968e6 + 49.104128e6,
+    ("limiter", 8): 293.320704e6 + 304.955392e6, ("limiter", 4): 168.422656e6 + 129.603584e6,
+    ("corr_flux", 8): 495.995904e6 + 206.604544e6, ("corr_flux", 4): 328.471296e6 + 95.712000e6,
+    ("corr_cell", 8): 468.177920e6 + 68.483840e6, ("corr_cell", 4): 275.880960e6 + 34.968064e6,
+    ("pred_flux", 8): 181.991680e6 + 188.046848e6, ("pred_flux", 4): 170.220032e6 + 84.814848e6,
+    ("pred_cell", 8): 343.044608e6 + 34.836480e6, ("pred_cell", 4): 192.598272e6 + 16.507392e6,
+    ("recon", 8): 259.743744e6 + 112.443136e6, ("recon", 4): 243.891968e6 + 49.104128e6,
 }
 # FP64 floating-point operations per launch on the same 64^3 launches (ncu
 # thread-instruction counts: 2 per DFMA, 1 per DADD and DMUL; this includes
 # the FMAs inside the compiler's divide and square-root sequences).  The plain
 # FP64 path is compared with the measured FP64 FMA peak (fvm_fp64_peak).
 NCU_FP64_FLOPS_64 = {
-    "limiter": 0.8236e9, "corr_flux": 1.4451e9, "corr_cell": 0.2531e9, "pred_flux": 1.4389e9,
-    "pred_cell": 0.2497e9, "recon": 1.0849e9,
+    "limiter": 0.8246e9, "corr_flux": 1.4514e9, "corr_cell": 0.2880e9, "pred_flux": 1.4389e9,
+    "pred_cell": 0.2143e9, "recon": 0.7879e9,
 }
 
 
