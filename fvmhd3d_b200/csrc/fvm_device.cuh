@@ -141,6 +141,7 @@ using namespace fvm;
 #ifndef FVM_SUMS_MINB
 #define FVM_SUMS_MINB 5
 #endif
+constexpr int LIMITER_SPLIT = 262144;  // cells above which k_limiter_st leaves the list to k_limiter
 constexpr int SUM_CELLS = 16384, SUM_BLOCK = 224;  // SUM_BLOCK: seven threads for each of 32 cells
 #ifndef FVM_GATHER_UNR
 #define FVM_GATHER_UNR 2
@@ -1089,24 +1090,34 @@ __global__ void __launch_bounds__(128, MINB) k_limiter(int n, Params P, const Sc
     const unsigned char *FVM_RESTRICT act, const double *FVM_RESTRICT tlast,
     const R *FVM_RESTRICT Wrec, R *FVM_RESTRICT tau, R *FVM_RESTRICT fst, const int *FVM_RESTRICT perm,
     const R *FVM_RESTRICT mnmx, const unsigned char *FVM_RESTRICT mz, const int *FVM_RESTRICT clist,
-    const R *FVM_RESTRICT lld) {
+    const R *FVM_RESTRICT lld, bool split) {
+  if (split && S->iscal[1] == n) return;
   limiter_dev<R, KH, MINB>(n, P, S, off, lnk, lfj, s12, geo, dr1, fflag, act, tlast, Wrec, tau, fst, perm, mnmx, mz, clist, lld, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 // The staged limiter: one block per CST cells.  In partial steps (clist not
 // null) a fixed grid, which stages the cells when every one is active and else
-// walks the involved-cell list, one thread per cell and primitive pair.
+// walks the involved-cell list, one thread per cell and primitive pair, or, when
+// split, leaves that to k_limiter, which returns when every cell is active.
+// One launch saves small steps 2 to 4 us; but the room that the staging takes
+// from the L1 cache costs a long walk more (1M-cell disk, FP64: 570K-cell steps
+// 2.07 ms against 1.50, 65K-cell steps 257 us against 193), so meshes of more
+// than LIMITER_SPLIT cells split it (64 individual steps of blasts, one
+// launch against two: 8.96 and 9.05 ms at 20^3, 14.05 and 14.18 at 40^3, 23.95
+// and 23.97 at 64^3).
 template <typename R, int KH, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_limiter_st(int n, Params P, const Sched *FVM_RESTRICT S,
     const int *FVM_RESTRICT off, const int *FVM_RESTRICT lnk, const int2 *FVM_RESTRICT lfj, const int2 *FVM_RESTRICT s12,
     const double4 *FVM_RESTRICT geo, const double4 *FVM_RESTRICT dr1, const unsigned char *FVM_RESTRICT fflag,
     const unsigned char *FVM_RESTRICT act, const double *FVM_RESTRICT tlast,
     const R *FVM_RESTRICT Wrec, R *FVM_RESTRICT tau, R *FVM_RESTRICT fst, const int *FVM_RESTRICT perm,
-    const R *FVM_RESTRICT mnmx, const unsigned char *FVM_RESTRICT mz, const int *FVM_RESTRICT clist, const R *FVM_RESTRICT lld) {
+    const R *FVM_RESTRICT mnmx, const unsigned char *FVM_RESTRICT mz, const int *FVM_RESTRICT clist, const R *FVM_RESTRICT lld,
+    bool split) {
   constexpr int CST = limiter_cst<KH>();
   extern __shared__ __align__(16) unsigned char lsm[];
   __shared__ int soff[2 * (CST + 1)];  // the cells' first links, and their first slots
   if (clist && S->iscal[1] != n) {
+    if (split) return;
     limiter_dev<R, KH, MINB>(n, P, S, off, lnk, lfj, s12, geo, dr1, fflag, act, tlast, Wrec, tau, fst, perm, mnmx, mz,
                              clist, lld, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
     return;

@@ -1034,6 +1034,11 @@ static int enq_begin(fvm_ctx *c) {
   return 0;
 }
 
+// Whether partial steps launch both limiters, each for its kind of step.
+static bool limiter_split(const fvm_ctx *c) {
+  return c->tune.lim_staged != 0 && c->use_flist && c->n > LIMITER_SPLIT;
+}
+
 // The staged limiter, instantiation MINB (resident blocks per SM).  A partial
 // step launches it on a grid of resident blocks, a global step on one block
 // per cell block.
@@ -1054,7 +1059,8 @@ static int limiter_st_launch(fvm_ctx *c) {
   const long long grid = c->use_flist ? std::min<long long>(ncb, (long long)MINB * c->sms) : ncb;
   k_limiter_st<R, KH, MINB><<<(unsigned)grid, 128, limiter_stage_bytes<R, KH>(), c->st>>>(
       c->n, c->P, d.S, d.off, d.lnk, d.lfj, d.s12, d.geo, d.dr1, d.fflag, d.act, d.tlast, (const R *)d.Wrec,
-      (R *)d.tau, (R *)d.fst, d.perm, (const R *)d.mnmx, d.mz, c->use_flist ? d.clist : nullptr, (const R *)d.lld);
+      (R *)d.tau, (R *)d.fst, d.perm, (const R *)d.mnmx, d.mz, c->use_flist ? d.clist : nullptr, (const R *)d.lld,
+      limiter_split(c));
   return 0;
 }
 }  // extern "C++"
@@ -1063,22 +1069,25 @@ static int enq_limiter(fvm_ctx *c) {
   Dev &d = c->d;
   kt_begin(c, KT_LIMITER);
   static_assert(FVM_CELL_PERM == 0, "the staged limiter maps threads to consecutive cells");
-  // The staged limiter when the autotuner picked it (partial steps choose
-  // between its staging and the list on the device), else the per-thread one.
+  // The staged limiter when the autotuner picked it, else the per-thread one.
+  // Partial steps choose on the device: by both launches, one of which returns
+  // at once (limiter_split), or inside the staged one.
   if (c->tune.lim_staged != 0) {
     BULK(({
       const int rc = c->use_flist ? limiter_st_launch<R, CellTune<R>::MINB_LIM>(c)
                                   : limiter_st_launch<R, CellTune<R>::MINB_LIM_G>(c);
       if (rc) return rc;
     }));
-  } else {
+  }
+  if (limiter_split(c)) LAUNCH_CHECK();
+  if (c->tune.lim_staged == 0 || limiter_split(c)) {
     const int bs = c->tune.bs_cell2;
 #define LIMITER_LIST(MB)                                                                                       \
   BULK(k_limiter<R, CellTune<R>::KH_LIM, MB>                                                                  \
        <<<sgrid(c, (long long)(10 / CellTune<R>::KH_LIM) * c->n, bs), bs, 0, c->st>>>(                         \
            c->n, c->P, d.S, d.off, d.lnk, d.lfj, d.s12, d.geo, d.dr1, d.fflag, d.act, d.tlast, (const R *)d.Wrec, \
            (R *)d.tau, (R *)d.fst, d.perm, (const R *)d.mnmx, d.mz, c->use_flist ? d.clist : nullptr,          \
-           (const R *)d.lld))
+           (const R *)d.lld, limiter_split(c)))
     if (c->use_flist) LIMITER_LIST(CellTune<R>::MINB_LIM);
     else LIMITER_LIST(CellTune<R>::MINB_LIM_G);
 #undef LIMITER_LIST
