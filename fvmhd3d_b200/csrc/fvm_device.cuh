@@ -37,7 +37,8 @@ struct Sched {
   int inc[2];  // incremental list building: [0] links of the active cells, [1] 1 when
                // this step's lists were built that way
   unsigned long long inc_steps;  // steps whose lists were built incrementally
-  int ff_all;                 // the face flags are those of every cell active (no partial step since)
+  int ff_all;                 // the last step ended with the face flags of every cell active
+  int ff_keep;                // ff_all as this step found it
   int ff_count;               // active faces of those flags
 };
 
@@ -241,7 +242,7 @@ __global__ void k_faceflags(int nf, const int2 *FVM_RESTRICT s12, unsigned char 
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   // a global step after one with every cell active: the flags stand (they
   // follow from the active cells and the boundary codes alone)
-  if (!bcount && S->ff_all && S->iscal[1] == n) {
+  if (!bcount && S->ff_keep && S->iscal[1] == n) {
     if (f == 0) *nface_active = S->ff_count;
     return;
   }
@@ -2786,6 +2787,8 @@ __global__ void k_sched_begin(Params P, Sched *S) {
   S->iscal[3] = 0;
   S->inc[0] = 0;
   S->inc[1] = 0;
+  S->ff_keep = S->ff_all;
+  S->ff_all = 0;  // until the step ends: one that fails midway leaves flags of its own
 }
 
 // The step's end in the scheduler's counters.
