@@ -1182,11 +1182,12 @@ static int enq_timesteps(fvm_ctx *c, int shared) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(c->st, &cs));
     if (cs != cudaStreamCaptureStatusNone) { c->err = "the timestep reduction needs eager steps"; return FVM_EINVAL; }
-    double &v = c->rb_host->dtmin;
-    CK(cudaMemcpyAsync(&v, &d.S->dtmin, sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(&c->rb_host->dtmin, &d.S->dtmin, sizeof(double), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
+    double v = c->rb_host->dtmin;  // the reduction's own: it may call this context, and pin_stage moves rb_host
     if (c->reduce(c->reduce_user, &v) != 0) { c->err = "the timestep reduction failed"; return FVM_EINVAL; }
-    CK(cudaMemcpyAsync(&d.S->dtmin, &v, sizeof(double), cudaMemcpyHostToDevice, c->st));
+    c->rb_host->dtmin = v;
+    CK(cudaMemcpyAsync(&d.S->dtmin, &c->rb_host->dtmin, sizeof(double), cudaMemcpyHostToDevice, c->st));
     CK(cudaStreamSynchronize(c->st));
   }
   if (!shared) {
