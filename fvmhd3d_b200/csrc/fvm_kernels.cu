@@ -193,6 +193,7 @@ struct fvm_ctx {
   // released with the context.
   void *ws = nullptr;
   size_t ws_bytes = 0;
+  std::vector<void *> ws_old;  // outgrown ones
   // Staging of small calls' host arrays (stage_of): one copy each way instead
   // of one per array.  stage is plain memory until pin_stage pins it.
   char *stage = nullptr, *stage_more = nullptr;
@@ -292,44 +293,60 @@ static int dalloc(fvm_ctx *c, T **p, size_t count) {
   return 0;
 }
 
-// Work space of one call, given back by ws_give after the call's last use on
-// the context's stream.  Up to kKeepBytes it is one buffer kept by the context
-// (allocating and trimming it cost a small call more than its work: 0.58 ms of
-// a gradient of 100 pairs); more is allocated for the call, so that a run that
-// holds most of the memory for its mesh does not hold this too.
-constexpr size_t kKeepBytes = 64u << 20;
-static int ws_take(fvm_ctx *c, void **p, size_t bytes) {
-  *p = nullptr;
-  if (bytes > kKeepBytes) {
-    CK(cudaMallocAsync(p, bytes, c->st));
-    return 0;
-  }
-  if (bytes > c->ws_bytes) {
-    if (c->ws) CK(cudaFreeAsync(c->ws, c->st));
-    c->ws = nullptr;
-    c->ws_bytes = 0;
-    CK(cudaMallocAsync(&c->ws, bytes, c->st));
-    c->ws_bytes = bytes;
-  }
-  *p = c->ws;
-  return 0;
-}
-static int ws_give(fvm_ctx *c, void *p) {
-  if (p && p != c->ws) CK(cudaFreeAsync(p, c->st));
-  return 0;
-}
-// Pinned host memory, or null (the caller goes on without); also while another
-// thread of the process captures a graph.
-static void *pinned(size_t bytes) {
+// Memory from one of the two allocation calls, or null (the caller goes on
+// without, or reports it); also while another thread of the process captures a
+// graph.
+template <typename F>
+static void *take_memory(F &&allocate, size_t bytes) {
   void *p = nullptr;
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
   cudaThreadExchangeStreamCaptureMode(&mode);
-  if (cudaMallocHost(&p, bytes) != cudaSuccess) {
+  if (allocate(&p, bytes) != cudaSuccess) {
     cudaGetLastError();
     p = nullptr;
   }
   cudaThreadExchangeStreamCaptureMode(&mode);
   return p;
+}
+// Pinned host memory.
+static void *pinned(size_t bytes) {
+  return take_memory([](void **p, size_t b) { return cudaMallocHost(p, b); }, bytes);
+}
+
+// Work space of one call, given back by ws_give after the call's last use on
+// the context's stream.  Up to kKeepBytes it is one buffer kept by the context
+// (allocating and trimming it cost a small call more than its work: 0.58 ms of
+// a gradient of 100 pairs); more is allocated for the call, so that a run that
+// holds most of the memory for its mesh does not hold this too: from the pool,
+// or for a caller whose call ends with a wait for its results alone (now) by
+// cudaMalloc, 0.6 ms less for the 96 MB of 300,000 faces (10.0 -> 9.4 ms).  The buffer
+// is made by cudaMalloc, a power of two long: as the pool's only block it cost
+// a context's first call 200 us, and its destruction the same (a batch of 40
+// faces 283 us against 96 with an allocation per call).  A buffer outgrown is
+// kept until the context goes, because freeing it would wait for every stream
+// of the device; with doubling sizes they add up to less than the last.
+constexpr size_t kKeepBytes = 64u << 20;
+static int ws_take(fvm_ctx *c, void **p, size_t bytes, bool now = false) {
+  *p = nullptr;
+  if (bytes > kKeepBytes) {
+    CK(now ? cudaMalloc(p, bytes) : cudaMallocAsync(p, bytes, c->st));
+    return 0;
+  }
+  if (bytes > c->ws_bytes) {
+    size_t room = 64u << 10;
+    while (room < bytes) room *= 2;
+    void *ws = take_memory([](void **q, size_t b) { return cudaMalloc(q, b); }, room);
+    if (!ws) { c->err = "work space: out of memory"; return FVM_ECUDA; }
+    if (c->ws) c->ws_old.push_back(c->ws);
+    c->ws = ws;
+    c->ws_bytes = room;
+  }
+  *p = c->ws;
+  return 0;
+}
+static int ws_give(fvm_ctx *c, void *p, bool now = false) {
+  if (p && p != c->ws) CK(now ? cudaFree(p) : cudaFreeAsync(p, c->st));
+  return 0;
 }
 // Pinning takes 2.5 ms whatever the size, as long as some hundred calls save by
 // it (a pageable copy is staged, and waits, by itself): the context's block
@@ -504,7 +521,8 @@ void fvm_destroy(fvm_ctx *c) {
   for (int k = 0; k < 2 * KT_COUNT; k++) cudaEventDestroy(c->kev[k]);
   if (c->gbar) cudaFree(c->gbar);
   if (c->gerr) cudaFree(c->gerr);
-  if (c->ws) cudaFreeAsync(c->ws, c->st);
+  if (c->ws) cudaFree(c->ws);
+  for (void *p : c->ws_old) cudaFree(p);
   if (c->stage_pinned) cudaFreeHost(c->stage);
   else free(c->stage);
   if (c->stage_more) cudaFreeHost(c->stage_more);
@@ -777,12 +795,12 @@ int fvm_init_problem(fvm_ctx *c, const double *W, const double *pos, const int *
   Dev &d = c->d;
   c->hs_ok = false;
   double *dW = nullptr;
-  int rc = ws_take(c, (void **)&dW, sizeof(double) * 10 * (size_t)n);
+  int rc = ws_take(c, (void **)&dW, sizeof(double) * 10 * (size_t)n, true);
   if (rc) return rc;
   cudaError_t e = cudaMemcpyAsync(dW, W, sizeof(double) * 10 * (size_t)n, cudaMemcpyHostToDevice, c->st);
-  if (e != cudaSuccess) { ws_give(c, dW); c->err = cudaGetErrorString(e); return FVM_ECUDA; }
+  if (e != cudaSuccess) { ws_give(c, dW, true); c->err = cudaGetErrorString(e); return FVM_ECUDA; }
   rc = enq_positions(c, pos, bnd);
-  if (rc) { ws_give(c, dW); return rc; }
+  if (rc) { ws_give(c, dW, true); return rc; }
   CK(cudaMemsetAsync(d.vel, 0, sizeof(double) * 3 * (size_t)n, c->st));
   CK(cudaMemsetAsync(d.tlast, 0, sizeof(double) * n, c->st));
 
@@ -804,7 +822,7 @@ int fvm_init_problem(fvm_ctx *c, const double *W, const double *pos, const int *
   LAUNCH_CHECK();
   double dtmin = 0.0;
   CK(cudaMemcpyAsync(&dtmin, &d.S->dtmin, sizeof(double), cudaMemcpyDeviceToHost, c->st));
-  if ((rc = ws_give(c, dW))) return rc;
+  if ((rc = ws_give(c, dW, true))) return rc;
   CK(cudaStreamSynchronize(c->st));
   if (c->reduce && c->reduce(c->reduce_user, &dtmin) != 0) {
     c->err = "fvm_init_problem: the timestep reduction failed";
@@ -1952,7 +1970,7 @@ int fvm_compute_flux(fvm_ctx *c, int nface, const double *wij, const double *Wi,
   // then psi, Bn, flux; the host's staging holds the same
   const size_t in = sizeof(double) * nf * 27, out = sizeof(double) * nf * 12;
   char *buf = nullptr;
-  int rc = ws_take(c, (void **)&buf, in + out);
+  int rc = ws_take(c, (void **)&buf, in + out, true);
   if (rc) return rc;
   double *dw = (double *)buf, *da = dw + 3 * nf, *db = da + 10 * nf, *dn = db + 10 * nf, *dp = dw + 27 * nf,
          *dB = dp + nf, *dF = dB + nf;
@@ -1973,7 +1991,7 @@ int fvm_compute_flux(fvm_ctx *c, int nface, const double *wij, const double *Wi,
   if (st) CK(cudaMemcpyAsync(st, dp, out, cudaMemcpyDeviceToHost, c->st));
   else
     for (const Part &p : outs) CK(cudaMemcpyAsync((void *)p.host, p.dev, p.bytes, cudaMemcpyDeviceToHost, c->st));
-  if ((rc = ws_give(c, buf))) return rc;
+  if ((rc = ws_give(c, buf, true))) return rc;
   CK(cudaStreamSynchronize(c->st));
   if (st)
     for (const Part &p : outs) memcpy((void *)p.host, st + ((char *)p.dev - (char *)dp), p.bytes);
