@@ -1553,14 +1553,19 @@ static int check_fused_errors(fvm_ctx *c) {
 // installs a mesh or state for each step never captures.
 constexpr int kGraphAfter = 8;
 static int step_graph(fvm_ctx *c, int shared);
+cudaError_t fvm_graph_instantiate(cudaGraphExec_t *exec, cudaGraph_t graph);
 
 int fvm_step(fvm_ctx *c, int shared) {
   if (!c || !c->have_state) { if (c) c->err = "fvm_step: no state"; return FVM_ENOMESH; }
   if (c->in_step) { c->err = "fvm_step: inside a step"; return FVM_EINVAL; }
   CK(cudaSetDevice(c->device));
   int rc = 0;
-  const bool replay = shared && !c->prof && !c->reduce && (c->graph[1] || ++c->eager_steps >= kGraphAfter);
-  if (replay && (rc = step_graph(c, shared))) return rc;
+  bool replay = shared && !c->prof && !c->reduce && (c->graph[1] || ++c->eager_steps >= kGraphAfter);
+  if (replay && step_graph(c, shared)) {  // no room for the graph: an eager step needs none
+    cudaGetLastError();
+    c->eager_steps = 0;
+    replay = false;
+  }
   c->hs_ok = false;
   CK(cudaEventRecord(c->ev0, c->st));
   if (replay) {
@@ -1667,6 +1672,17 @@ int fvm_step_host(fvm_ctx *c, int shared, unsigned long long tsys_ticks, double 
   return c->hS.iscal[1];
 }
 
+// The one call of a captured step that takes memory of its own; a symbol of
+// the library, so that a test can stand a failing one in its place.  Also while
+// another thread of the process captures a graph.
+__attribute__((noinline)) cudaError_t fvm_graph_instantiate(cudaGraphExec_t *exec, cudaGraph_t graph) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  const cudaError_t e = cudaGraphInstantiate(exec, graph, 0);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return e;
+}
+
 // The captured step of the mode, made on first use.  Per-kernel profiling is
 // not recorded in it.
 static int step_graph(fvm_ctx *c, int shared) {
@@ -1685,7 +1701,7 @@ static int step_graph(fvm_ctx *c, int shared) {
   c->prof = prof;
   if (rc) { if (gr) cudaGraphDestroy(gr); return rc; }
   if (e != cudaSuccess) { c->err = std::string("graph capture: ") + cudaGetErrorString(e); return FVM_ECUDA; }
-  e = cudaGraphInstantiate(&c->graph[g], gr, 0);
+  e = fvm_graph_instantiate(&c->graph[g], gr);
   cudaGraphDestroy(gr);
   if (e != cudaSuccess) { c->graph[g] = nullptr; c->err = std::string("graph instantiate: ") + cudaGetErrorString(e); return FVM_ECUDA; }
   return 0;
