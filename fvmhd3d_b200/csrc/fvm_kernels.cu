@@ -188,7 +188,7 @@ struct fvm_ctx {
     double dtmin;
   } *rb_host = nullptr;
   bool hs_ok = false;  // hS is the device's: nothing was enqueued since it was read
-  int eager_steps = 0;  // consecutive eager global steps of this state (fvm_step)
+  int eager_steps = 0;  // eager global steps since the last change of mesh or settings (fvm_step)
   // Work space of calls on host arrays (ws_take), kept up to kKeepBytes and
   // released with the context.
   void *ws = nullptr;
@@ -1547,10 +1547,12 @@ static int check_fused_errors(fvm_ctx *c) {
   return FVM_ECUDA;
 }
 
-// Global steps of one state replay the captured step from the
+// Global steps of one mesh and its settings replay the captured step from the
 // kGraphAfter-th call on, when its capture has paid off: the launches of an
-// eager step take longer than the kernels of a small mesh.  A host that
-// installs a mesh or state for each step never captures.
+// eager step take longer than the kernels of a small mesh.  (Partial steps in
+// between do not count, and a new state keeps the graph: it holds no state.)
+// A host that installs a mesh, positions by fvm_init_problem or settings for
+// each step never captures.
 constexpr int kGraphAfter = 8;
 static int step_graph(fvm_ctx *c, int shared);
 cudaError_t fvm_graph_instantiate(cudaGraphExec_t *exec, cudaGraph_t graph);
@@ -1696,7 +1698,8 @@ static int step_graph(fvm_ctx *c, int shared) {
   CK(be);
   const long long l0 = c->launches;
   const int rc = enq_step(c, shared);
-  c->graph_launches[g] = c->launches - l0;
+  c->graph_launches[g] = c->launches - l0;  // counted when it runs
+  c->launches = l0;
   cudaError_t e = cudaStreamEndCapture(c->st, &gr);
   c->prof = prof;
   if (rc) { if (gr) cudaGraphDestroy(gr); return rc; }
@@ -1720,7 +1723,10 @@ int fvm_run(fvm_ctx *c, int nsteps, int shared, long long *faces_out) {
   const unsigned long long a0 = c->hS.nactive_total, f0 = c->hS.nfaces_total;
   c->hs_ok = false;
   CK(cudaEventRecord(c->ev0, c->st));
-  for (int k = 0; k < nsteps; k++) CK(cudaGraphLaunch(c->graph[shared ? 1 : 0], c->st));
+  for (int k = 0; k < nsteps; k++) {
+    CK(cudaGraphLaunch(c->graph[shared ? 1 : 0], c->st));
+    c->launches += c->graph_launches[shared ? 1 : 0];
+  }
   CK(cudaEventRecord(c->ev1, c->st));
   if ((rc = read_sched(c))) return rc;
   if ((rc = check_fused_errors(c))) return rc;

@@ -384,7 +384,9 @@ int fvm_last_adjust_stats(const fvm_ctx *c, int *dirty_sites, int *replays, int 
  * that FP64-bound kernels are compared with (after fvm_set_mesh).  No
  * counterpart in the reference (a measurement aid). */
 int fvm_fp64_peak(fvm_ctx *c, double *flops_per_s);
-/* Number of kernels this context has launched so far. */
+/* Number of kernels this context has launched so far, those of replayed steps
+ * included (a replayed individual step counts the kernels of both branches of
+ * its graph's choices, and the body of the adjust_timesteps loop once). */
 long long fvm_launch_count(const fvm_ctx *c);
 /* Per-kernel CUDA-event timing: on != 0 enables it and clears the totals. */
 int fvm_set_profiling(fvm_ctx *c, int on);
