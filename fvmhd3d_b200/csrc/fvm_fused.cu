@@ -248,17 +248,23 @@ namespace fvm {
 
 int fused_step_blocks_per_sm(bool fp32) { return fp32 ? blocks_per_sm<float>() : blocks_per_sm<double>(); }
 
-cudaError_t fused_step_enqueue(const FusedStep &a, bool fp32, int grid, cudaStream_t st) {
-  // The grid is the kernel's occupancy limit times the SM count and the
-  // launch is the only work on its stream, so every block is resident at
-  // once and the grid barriers can complete; were some not resident, the
-  // bounded barriers would end the launch with err bit 1, not hang.
+cudaError_t fused_step_enqueue(const FusedStep &a, bool fp32, int grid, bool cooperative, cudaStream_t st) {
+  // A cooperative launch starts when every block of the grid can be resident
+  // and not before, whatever other streams and contexts run on the device, so
+  // the grid barriers complete.  (Two plain launches of this size, by two
+  // contexts, could each hold part of the SMs and wait for blocks that no
+  // longer fit.)
   if (grid <= 0) return cudaErrorInvalidConfiguration;
-  if (fp32)
-    k_rung_step<float><<<grid, 128, 0, st>>>(a);
-  else
-    k_rung_step<double><<<grid, 128, 0, st>>>(a);
-  return cudaGetLastError();
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeCooperative;
+  attr.val.cooperative = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(128);
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = cooperative ? 1 : 0;
+  return fp32 ? cudaLaunchKernelEx(&cfg, k_rung_step<float>, a) : cudaLaunchKernelEx(&cfg, k_rung_step<double>, a);
 }
 
 }  // namespace fvm

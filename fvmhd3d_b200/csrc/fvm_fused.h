@@ -20,9 +20,11 @@ struct FusedStep {
 // Enqueues one persistent launch of the partial step on `st`: every stage
 // from the slope limiter to the reconstruction over the step's involved
 // cells and active faces, with grid-wide barriers between the stages.  grid:
-// at most fused_step_blocks_per_sm times the SM count.  Returns the CUDA error
-// of the launch.
-cudaError_t fused_step_enqueue(const FusedStep &a, bool fp32, int grid, cudaStream_t st);
+// at most fused_step_blocks_per_sm times the SM count.  cooperative: false only
+// where the device cannot launch cooperatively; the grid is then one block per
+// SM, which leaves room for the grids of other contexts.  Returns the CUDA
+// error of the launch.
+cudaError_t fused_step_enqueue(const FusedStep &a, bool fp32, int grid, bool cooperative, cudaStream_t st);
 
 // Blocks of the persistent kernel resident per SM.
 int fused_step_blocks_per_sm(bool fp32);

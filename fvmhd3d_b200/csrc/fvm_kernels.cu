@@ -225,6 +225,7 @@ struct fvm_ctx {
   // -1: automatic, see inc_limit)
   int inc_max = -1;
   int fused_bpsm = 0;          // its resident blocks per SM (queried outside capture)
+  bool fused_coop = false;     // its launch is cooperative (a device shared through MPS has no such launches)
   // the reduction of the timestep minimum over ranks (fvm_set_reduce)
   fvm_reduce_fn reduce = nullptr;
   void *reduce_user = nullptr;
@@ -506,6 +507,11 @@ fvm_ctx *fvm_create(const fvm_params *p, int device) {
   }
   c->rb_host = reinterpret_cast<fvm_ctx::ReadBack *>(c->stage + kStageBytes);
   c->fused_bpsm = fused_step_blocks_per_sm(c->fp32);
+  int coop = 0, mps = 0;
+  if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess) coop = 0;
+  if (cudaDeviceGetAttribute(&mps, cudaDevAttrMpsEnabled, device) != cudaSuccess) mps = 0;
+  cudaGetLastError();
+  c->fused_coop = coop && !mps;
   return c;
 }
 
@@ -1375,11 +1381,16 @@ static int enq_stages(fvm_ctx *c, int shared) {
 }
 
 // Blocks per SM of the persistent rung kernel's grid (at most its resident
-// limit): a step it runs involves few cells, and fewer blocks make each grid
-// barrier cheaper.
+// limit), for the steps of many involved cells; those of few let one per SM
+// work (k_rung_step).  One where the launch cannot be cooperative.
 #ifndef FVM_FUSED_BPSM
 #define FVM_FUSED_BPSM 4
 #endif
+static cudaError_t launch_fused(fvm_ctx *c, cudaStream_t st) {
+  const FusedStep a = {c->P, c->d, c->lb, c->n, c->nf, c->sms, c->gbar, c->gerr};
+  const int per = c->fused_coop ? std::min(c->fused_bpsm, FVM_FUSED_BPSM) : 1;
+  return fused_step_enqueue(a, c->fp32, per * c->sms, c->fused_coop, st);
+}
 
 // Sets the branch of a captured partial step: the persistent rung kernel
 // when the step involves at most max_cells cells (and not every cell), else
@@ -1412,11 +1423,10 @@ static int enq_fused_or_stages(fvm_ctx *c) {
   cudaGraphNode_t cn;
   CK(cudaGraphAddNode(&cn, g, deps, nd, &cp));
   cudaGraph_t body_fused = cp.conditional.phGraph_out[0], body_stages = cp.conditional.phGraph_out[1];
-  // if: the persistent kernel (one plain kernel node), captured from the
+  // if: the persistent kernel (one cooperative kernel node), captured from the
   // auxiliary stream
   CK(cudaStreamBeginCaptureToGraph(c->aux, body_fused, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-  const FusedStep a = {c->P, c->d, c->lb, c->n, c->nf, c->sms, c->gbar, c->gerr};
-  const cudaError_t le = fused_step_enqueue(a, c->fp32, std::min(c->fused_bpsm, FVM_FUSED_BPSM) * c->sms, c->aux);
+  const cudaError_t le = launch_fused(c, c->aux);
   cudaGraph_t done = nullptr;
   const cudaError_t ee = cudaStreamEndCapture(c->aux, &done);
   CK(le);
@@ -1458,8 +1468,7 @@ static int enq_step(fvm_ctx *c, int shared) {
     const int ninv = c->rb_host->counts[0];
     if (ninv <= c->fused_max && ninv < c->n) {
       kt_begin(c, KT_FUSED);
-      const FusedStep a = {c->P, c->d, c->lb, c->n, c->nf, c->sms, c->gbar, c->gerr};
-      CK(fused_step_enqueue(a, c->fp32, std::min(c->fused_bpsm, FVM_FUSED_BPSM) * c->sms, c->st));
+      CK(launch_fused(c, c->st));
       c->launches += 1;
       kt_end(c, KT_FUSED);
       rc = 0;
