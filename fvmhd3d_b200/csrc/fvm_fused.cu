@@ -28,10 +28,6 @@ constexpr int kCellGroup = 8;
 // cell, so a cell takes 20 lanes).
 constexpr int kLimGroup = 4;
 
-// Polls of a grid barrier wait before it gives up (about 100 ns each): far
-// above the longest stage of a step this kernel runs (the sequential
-// adjust_timesteps sweep over at most its involved cells).
-constexpr long long kBarrierPolls = 1ll << 24;
 #ifndef FVM_FUSED_WIDE
 #define FVM_FUSED_WIDE 2048
 #endif
@@ -43,42 +39,7 @@ __device__ __forceinline__ unsigned load_acquire(const unsigned *p) {
   return v;
 }
 
-// Grid-wide barrier over the nblocks working blocks of the launch (the
-// first nblocks; the others have returned).  bar[0] counts arrivals, zero at
-// the start of the launch: thread 0 of each block arrives after a release
-// fence and waits, with bounded polls, until the count covers every block's
-// passage of this barrier (`passed` of them before it).  One atomic and the
-// polls are all a barrier costs; the counters are cleared at the end of the
-// launch (grid_done).  Returns false on every thread of the block if the wait
-// gave up (err bit 1 set).
-__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned &passed, int *err, unsigned nblocks) {
-  __syncthreads();
-  passed++;
-  int ok = 1;
-  if (threadIdx.x == 0) {
-    const unsigned target = passed * nblocks;
-    __threadfence();
-    atomicAdd(&bar[0], 1u);
-    long long it = 0;
-    while (load_acquire(&bar[0]) < target) {
-      if (++it > kBarrierPolls) {
-        atomicOr(err, 1);
-        ok = 0;
-        break;
-      }
-      if (it > 4096) __nanosleep(64);  // short waits spin; long ones back off
-    }
-    __threadfence();
-  }
-  return __syncthreads_and(ok) != 0;
-}
-// After a block's last barrier: the last block of all clears the counters.
-__device__ __forceinline__ void grid_done(unsigned *bar, unsigned nblocks) {
-  if (threadIdx.x == 0 && atomicAdd(&bar[1], 1u) == nblocks - 1) {
-    bar[0] = 0u;
-    bar[1] = 0u;
-  }
-}
+#include "grid_barrier.cuh"
 
 __device__ __forceinline__ int vload(const int *p) { return *reinterpret_cast<const volatile int *>(p); }
 
@@ -92,6 +53,7 @@ __global__ void __launch_bounds__(128, FVM_FLUX_MINB) k_rung_step(FusedStep a) {
   const Dev &d = a.d;
   Sched *S = d.S;
   const int n = a.n, nf = a.nf;
+  if (grid_failed(a.gerr)) return;
   // The stages of a small step are bound by the latency of each thread's walk
   // over its cell's faces, so more threads beat cheaper barriers: one block
   // per SM works however few the cells (one block per 64 involved cells
@@ -109,7 +71,7 @@ __global__ void __launch_bounds__(128, FVM_FLUX_MINB) k_rung_step(FusedStep a) {
 #define FVM_GRID_SYNC() \
   if (!grid_barrier(a.gbar, passed, a.gerr, nwork)) return
   // the work arrays of adjust_timesteps start cleared for the step's
-  // involved cells (the separate-kernel step clears them for every cell).
+  // involved cells (in a step of stage kernels k_timestep clears them).
   // Every entry this step writes or reads is an involved cell's: marks and
   // work lists go to active cells and their neighbours, and the replays
   // below walk the involved cells only.
