@@ -320,12 +320,15 @@ static void *pinned(size_t bytes) {
 // a gradient of 100 pairs); more is allocated for the call, so that a run that
 // holds most of the memory for its mesh does not hold this too: from the pool,
 // or for a caller whose call ends with a wait for its results alone (now) by
-// cudaMalloc, 0.6 ms less for the 96 MB of 300,000 faces (10.0 -> 9.4 ms).  The buffer
-// is made by cudaMalloc, a power of two long: as the pool's only block it cost
-// a context's first call 200 us, and its destruction the same (a batch of 40
-// faces 283 us against 96 with an allocation per call).  A buffer outgrown is
-// kept until the context goes, because freeing it would wait for every stream
-// of the device; with doubling sizes they add up to less than the last.
+// cudaMalloc, 0.6 ms less for the 96 MB of 300,000 faces (10.0 -> 9.4 ms).  The
+// buffer is made by cudaMalloc: as the pool's only block it cost a context's
+// first call 200 us, and its destruction the same (a batch of 40 faces 283 us
+// against 96 with an allocation per call).  A first buffer is as long as asked
+// (rounded up to 1 MB, that of 3,000 faces, 0.94 MB, cost 0.5 to 4 ms, because
+// the driver no longer carves it from a block it has), a larger one at least
+// twice the last.  A buffer outgrown is kept until the context goes, because
+// freeing it would wait for every stream of the device; with doubling sizes
+// they add up to less than the last.
 constexpr size_t kKeepBytes = 64u << 20;
 static int ws_take(fvm_ctx *c, void **p, size_t bytes, bool now = false) {
   *p = nullptr;
@@ -334,8 +337,7 @@ static int ws_take(fvm_ctx *c, void **p, size_t bytes, bool now = false) {
     return 0;
   }
   if (bytes > c->ws_bytes) {
-    size_t room = 64u << 10;
-    while (room < bytes) room *= 2;
+    const size_t room = std::max(bytes, std::min(2 * c->ws_bytes, kKeepBytes));
     void *ws = take_memory([](void **q, size_t b) { return cudaMalloc(q, b); }, room);
     if (!ws) { c->err = "work space: out of memory"; return FVM_ECUDA; }
     if (c->ws) c->ws_old.push_back(c->ws);
