@@ -22,6 +22,7 @@
 #include <cmath>
 #include <cstdint>
 #include <mutex>
+#include <new>
 #include <cstdio>
 #include <cstring>
 #include <climits>
@@ -181,12 +182,14 @@ struct fvm_ctx {
   // one captured step per mode (shared / individual), replayed by fvm_run
   cudaGraphExec_t graph[2];
   Sched hS;  // host copy of the device scheduler, refreshed after synchronisation
-  // what a synchronisation reads back, behind the staging (stage)
+  // what a synchronisation reads back: into plain memory, after kPinReads of
+  // them into pinned memory (read_sched)
   struct ReadBack {
     Sched S;
     int gerr, counts[2];
     double dtmin;
-  } *rb_host = nullptr;
+  } back_plain = {}, *back = &back_plain;
+  int reads = 0;
   bool hs_ok = false;  // hS is the device's: nothing was enqueued since it was read
   int eager_steps = 0;  // eager global steps since the last change of mesh or settings (fvm_step)
   // Work space of calls on host arrays (ws_take), kept up to kKeepBytes and
@@ -195,7 +198,7 @@ struct fvm_ctx {
   size_t ws_bytes = 0;
   std::vector<void *> ws_old;  // outgrown ones
   // Staging of small calls' host arrays (stage_of): one copy each way instead
-  // of one per array.  stage is plain memory until pin_stage pins it.
+  // of one per array.
   char *stage = nullptr, *stage_more = nullptr;
   bool stage_pinned = false;
   int small_calls = 0, staged_calls = 0;
@@ -351,34 +354,33 @@ static int ws_give(fvm_ctx *c, void *p, bool now = false) {
   if (p && p != c->ws) CK(now ? cudaFree(p) : cudaFreeAsync(p, c->st));
   return 0;
 }
-// Pinning takes 2.5 ms whatever the size, as long as some hundred calls save by
-// it (a pageable copy is staged, and waits, by itself): the context's block
-// (kStageBytes of staging and what a synchronisation reads back) is plain
-// memory until kPinAfter calls have used it, so that creating a context does
-// not pay for it.  Called where no copy of the block is in flight.
+// Staging of calls on small host arrays, pinned only for contexts that make
+// many of them: pinning takes 1.2 to 4 ms whatever the size, and freeing it
+// again 0.4.  Batches of up to kStageBytes go through plain memory first (one
+// copy each way instead of eight, 83 -> 46 us for 40 faces), then through
+// pinned memory (30 us) from the kPinAfter-th on, when what the staging has
+// saved pays for it.  Batches of up to kStageMore gain by pinned memory alone
+// (3,000 faces 178 -> 115 us) and until then are copied as they are; after
+// kStageAfter of them pinning costs 4% of what they took, after 32, where the
+// savings would catch up soonest, a context that stopped there took 1.3 times
+// as long.
 constexpr size_t kStageBytes = 64u << 10, kStageMore = 1u << 20;
-constexpr int kPinAfter = 64, kStageAfter = 32;
-static void pin_stage(fvm_ctx *c) {
-  if (c->stage_pinned || c->small_calls >= kPinAfter || ++c->small_calls < kPinAfter) return;
-  char *p = (char *)pinned(kStageBytes + sizeof(*c->rb_host));
-  if (!p) return;
-  memcpy(p + kStageBytes, c->rb_host, sizeof(*c->rb_host));
-  free(c->stage);
-  c->stage = p;
-  c->rb_host = reinterpret_cast<fvm_ctx::ReadBack *>(p + kStageBytes);
-  c->stage_pinned = true;
-}
-// Null where the arrays are copied as they are.  Up to kStageBytes the staging
-// is part of the context's one block; a call of up to kStageMore saves more by
-// pinned staging (a batch of 3,000 faces 170 -> 95 us), so a context pins that
-// much when it has made kStageAfter such calls.
+constexpr int kPinAfter = 128, kStageAfter = 256;
+// Null where the arrays are copied as they are.
 static char *stage_of(fvm_ctx *c, size_t bytes) {
   if (bytes <= kStageBytes) {
-    pin_stage(c);
+    if (!c->stage_pinned && c->small_calls < kPinAfter && ++c->small_calls == kPinAfter) {
+      if (char *p = (char *)pinned(kStageBytes)) {
+        free(c->stage);
+        c->stage = p;
+        c->stage_pinned = true;
+      }
+    }
     return c->stage;
   }
   if (bytes > kStageMore) return nullptr;
-  if (!c->stage_more && ++c->staged_calls == kStageAfter) c->stage_more = (char *)pinned(kStageMore);
+  if (!c->stage_more && c->staged_calls < kStageAfter && ++c->staged_calls == kStageAfter)
+    c->stage_more = (char *)pinned(kStageMore);
   return c->stage_more;
 }
 
@@ -503,11 +505,10 @@ fvm_ctx *fvm_create(const fvm_params *p, int device) {
   if (cudaStreamCreateWithFlags(&c->aux, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&c->gbar, 2 * sizeof(unsigned)) != cudaSuccess || cudaMalloc(&c->gerr, sizeof(int)) != cudaSuccess ||
       cudaMemset(c->gerr, 0, sizeof(int)) != cudaSuccess || cudaMemset(c->gbar, 0, 2 * sizeof(unsigned)) != cudaSuccess ||
-      !(c->stage = (char *)calloc(1, kStageBytes + sizeof(*c->rb_host)))) {
+      !(c->stage = (char *)malloc(kStageBytes))) {
     fvm_destroy(c);
     return nullptr;
   }
-  c->rb_host = reinterpret_cast<fvm_ctx::ReadBack *>(c->stage + kStageBytes);
   c->fused_bpsm = fused_step_blocks_per_sm(c->fp32);
   int coop = 0, mps = 0;
   if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess) coop = 0;
@@ -534,6 +535,7 @@ void fvm_destroy(fvm_ctx *c) {
   if (c->stage_pinned) cudaFreeHost(c->stage);
   else free(c->stage);
   if (c->stage_more) cudaFreeHost(c->stage_more);
+  if (c->back != &c->back_plain) cudaFreeHost(c->back);
   cudaEventDestroy(c->ev0);
   cudaEventDestroy(c->ev1);
   if (c->aux) cudaStreamDestroy(c->aux);
@@ -735,14 +737,20 @@ int fvm_set_mesh(fvm_ctx *c, int ncell, int nface, const int *s1, const int *s2,
 }
 
 // Synchronise and refresh the host copy of the scheduler (and, with the
-// persistent rung kernel on, of its error bits).
+// persistent rung kernel on, of its error bits).  Pinned memory saves 2 to 4 us
+// of a read (a 6^3 step with its state's read 135 -> 133 us, a step by stage
+// calls 1.317 -> 1.305 ms) and takes 1.2 to 4 ms to make, so a context does with
+// plain memory for its first kPinReads.
+constexpr int kPinReads = 128;
 static int read_sched(fvm_ctx *c) {
-  pin_stage(c);
-  c->rb_host->gerr = 0;
-  CK(cudaMemcpyAsync(&c->rb_host->S, c->d.S, sizeof(Sched), cudaMemcpyDeviceToHost, c->st));
-  if (c->fused_max > 0) CK(cudaMemcpyAsync(&c->rb_host->gerr, c->gerr, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+  if (c->reads < kPinReads && ++c->reads == kPinReads) {
+    if (void *p = pinned(sizeof(*c->back))) c->back = new (p) fvm_ctx::ReadBack(c->back_plain);
+  }
+  c->back->gerr = 0;
+  CK(cudaMemcpyAsync(&c->back->S, c->d.S, sizeof(Sched), cudaMemcpyDeviceToHost, c->st));
+  if (c->fused_max > 0) CK(cudaMemcpyAsync(&c->back->gerr, c->gerr, sizeof(int), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
-  c->hS = c->rb_host->S;
+  c->hS = c->back->S;
   c->hs_ok = true;
   c->tsysU = c->hS.tsysU;
   c->t_global = c->hS.t_global;
@@ -1041,7 +1049,7 @@ static int enq_begin(fvm_ctx *c) {
     rc = enq_lists_choice(c);
   } else if (inc && cs == cudaStreamCaptureStatusNone) {
     // an eager step makes the same choice on the host
-    int *cnt = c->rb_host->counts;
+    int *cnt = c->back->counts;
     CK(cudaMemcpyAsync(&cnt[0], &d.S->iscal[1], sizeof(int), cudaMemcpyDeviceToHost, c->st));
     CK(cudaMemcpyAsync(&cnt[1], &d.S->inc[0], sizeof(int), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
@@ -1208,12 +1216,12 @@ static int enq_timesteps(fvm_ctx *c, int shared) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(c->st, &cs));
     if (cs != cudaStreamCaptureStatusNone) { c->err = "the timestep reduction needs eager steps"; return FVM_EINVAL; }
-    CK(cudaMemcpyAsync(&c->rb_host->dtmin, &d.S->dtmin, sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(&c->back->dtmin, &d.S->dtmin, sizeof(double), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    double v = c->rb_host->dtmin;  // the reduction's own: it may call this context, and pin_stage moves rb_host
+    double v = c->back->dtmin;  // the reduction's own: it may call this context
     if (c->reduce(c->reduce_user, &v) != 0) { c->err = "the timestep reduction failed"; return FVM_EINVAL; }
-    c->rb_host->dtmin = v;
-    CK(cudaMemcpyAsync(&d.S->dtmin, &c->rb_host->dtmin, sizeof(double), cudaMemcpyHostToDevice, c->st));
+    c->back->dtmin = v;
+    CK(cudaMemcpyAsync(&d.S->dtmin, &c->back->dtmin, sizeof(double), cudaMemcpyHostToDevice, c->st));
     CK(cudaStreamSynchronize(c->st));
   }
   if (!shared) {
@@ -1465,9 +1473,9 @@ static int enq_step(fvm_ctx *c, int shared) {
   } else if (fusable && cs == cudaStreamCaptureStatusNone) {
     // an eager step makes the same choice on the host, from the involved-cell
     // count the step's list building left on the device
-    CK(cudaMemcpyAsync(c->rb_host->counts, &c->d.S->ninv, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(c->back->counts, &c->d.S->ninv, sizeof(int), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    const int ninv = c->rb_host->counts[0];
+    const int ninv = c->back->counts[0];
     if (ninv <= c->fused_max && ninv < c->n) {
       kt_begin(c, KT_FUSED);
       CK(launch_fused(c, c->st));
@@ -1524,9 +1532,9 @@ int fvm_compute_timesteps(fvm_ctx *c, int shared, double *dt_min_out) {
   int rc = enq_timesteps(c, shared);
   if (rc) return rc;
   if (dt_min_out) {
-    CK(cudaMemcpyAsync(&c->rb_host->dtmin, &c->d.S->dtmin, sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(&c->back->dtmin, &c->d.S->dtmin, sizeof(double), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    *dt_min_out = c->rb_host->dtmin;
+    *dt_min_out = c->back->dtmin;
   }
   return 0;
 }
@@ -1551,7 +1559,7 @@ int fvm_end_step(fvm_ctx *c, int shared) {
 // results are then incomplete): reported, and the barrier cleared.
 // (as of the last read_sched)
 static int check_fused_errors(fvm_ctx *c) {
-  if (!c->rb_host->gerr) return 0;
+  if (!c->back->gerr) return 0;
   cudaMemset(c->gbar, 0, 2 * sizeof(unsigned));
   cudaMemset(c->gerr, 0, sizeof(int));
   c->err = "a grid barrier of the persistent rung kernel timed out";

@@ -43,3 +43,34 @@ def test_first_calls_leave_the_pool_alone(faces):
         if want_f is not None:
             assert np.array_equal(y, want_y) and all(np.array_equal(a, b, equal_nan=True) for a, b in zip(f, want_f))
         want_f, want_y = f, y
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("faces,calls", [(40, 130), (400, 260)])
+def test_batches_around_the_pinning_of_their_staging(faces, calls):
+    """The staging of batches of up to 64 KB is pinned after 128 of them, that
+    of batches of up to 1 MB after 256; the results stay the first call's."""
+    s = F.System()
+    args = face_batch(faces, seed=6)
+    want = s.compute_flux(*args)
+    for _ in range(calls):
+        for a, b in zip(s.compute_flux(*args), want):
+            assert np.array_equal(a, b, equal_nan=True)
+
+
+@pytest.mark.gpu
+def test_steps_around_the_pinning_of_what_they_read():
+    """What a step reads back goes to pinned memory after 128 of them."""
+    m = F.build_periodic(F.jittered_lattice(4, 0.1, seed=5), 1.0)
+    W = F.problems.blast(m.pos)
+    s, once = F.System(), F.System()
+    for x in (s, once):
+        x.set_mesh(m)
+        x.init_problem(W)
+    for k in range(150):
+        assert s.step(shared=True) == m.ncell and s.active_face_count() == m.nface
+    once.run(150, shared=True)
+    assert s.clock() == once.clock()
+    a, b = s.get_state(), once.get_state()
+    for k in a:
+        assert np.array_equal(a[k], b[k]), k

@@ -1,6 +1,7 @@
-"""A timestep reduction that makes calls of its own on the context, past the
-64th small one, which moves the context's staging to pinned memory: the step
-continues with the reduction's value, and nobody else's memory is written."""
+"""A timestep reduction that makes calls of its own on the context, more than
+the number after which the staging of small batches moves to pinned memory:
+the step continues with the reduction's value, and nobody else's memory is
+written."""
 import numpy as np
 import pytest
 
@@ -14,7 +15,7 @@ def test_reduction_that_moves_the_staging():
     W = F.problems.blast(m.pos)
     args = face_batch(40, seed=6)
     held, out = [], []
-    for calls in (0, 70):
+    for calls in (0, 150):
         s = F.System()
         s.set_mesh(m)
         s.init_problem(W)
