@@ -142,7 +142,7 @@ using namespace fvm;
 #ifndef FVM_SUMS_MINB
 #define FVM_SUMS_MINB 5
 #endif
-constexpr int LIMITER_SPLIT = 262144;  // cells above which k_limiter_st leaves the list to k_limiter
+constexpr int LIMITER_SPLIT = 65536;  // cells above which k_limiter_st leaves the list to k_limiter
 constexpr int SUM_CELLS = 16384, SUM_BLOCK = 224;  // SUM_BLOCK: seven threads for each of 32 cells
 #ifndef FVM_GATHER_UNR
 #define FVM_GATHER_UNR 2
@@ -1103,9 +1103,12 @@ __global__ void __launch_bounds__(128, MINB) k_limiter(int n, Params P, const Sc
 // One launch saves small steps 2 to 4 us; but the room that the staging takes
 // from the L1 cache costs a long walk more (1M-cell disk, FP64: 570K-cell steps
 // 2.07 ms against 1.50, 65K-cell steps 257 us against 193), so meshes of more
-// than LIMITER_SPLIT cells split it (64 individual steps of blasts, one
-// launch against two: 8.96 and 9.05 ms at 20^3, 14.05 and 14.18 at 40^3, 23.95
-// and 23.97 at 64^3).
+// than LIMITER_SPLIT cells split it.  64 individual steps, one launch against
+// two, FP64 (FP32), ms: blasts of 20^3 8.96 and 9.05, 40^3 14.05 and 14.18,
+// 48^3 18.5 and 18.2 (17.5 and 17.5), 80^3 44.1 and 43.0 (36.9 and 36.4); disks
+// of 60K cells 13.6 to 14.0 and 13.7 (13.4 and 13.3), 120K 21.6 and 20.8 (19.6
+// and 18.5 to 19.1), 250K 36.1 to 36.7 and 34.3 to 34.9 (31.2 and 29.8 to
+// 30.3), 1M 101 and 93 (79.8 and 76.1).
 template <typename R, int KH, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_limiter_st(int n, Params P, const Sched *FVM_RESTRICT S,
     const int *FVM_RESTRICT off, const int *FVM_RESTRICT lnk, const int2 *FVM_RESTRICT lfj, const int2 *FVM_RESTRICT s12,
