@@ -68,17 +68,17 @@ def kernel_bytes(name, N, F, prec_bytes=8):
 
 # DRAM bytes (read + write) per launch measured by ncu on the 64^3 blast
 # (262144 cells, 2085347 faces; profiles/global_step_kernels_blast64_fp64.md and
-# cell_and_face_kernels_blast64_fp32_full.md; FP64 cell passes with their pass of
+# global_step_kernels_blast64_fp32.md; FP64 cell passes with their pass of
 # sums), per face; a launch on another mesh of the same kind moves these bytes times
 # its face count.
 NCU_FACES_64 = 2085347
 NCU_TRAFFIC_64 = {
-    ("limiter", 8): 293.320704e6 + 304.955392e6, ("limiter", 4): 168.422656e6 + 129.603584e6,
-    ("corr_flux", 8): 495.995904e6 + 206.604544e6, ("corr_flux", 4): 328.471296e6 + 95.712000e6,
-    ("corr_cell", 8): 468.177920e6 + 68.483840e6, ("corr_cell", 4): 275.880960e6 + 34.968064e6,
-    ("pred_flux", 8): 181.991680e6 + 188.046848e6, ("pred_flux", 4): 170.220032e6 + 84.814848e6,
-    ("pred_cell", 8): 343.044608e6 + 34.836480e6, ("pred_cell", 4): 192.598272e6 + 16.507392e6,
-    ("recon", 8): 259.743744e6 + 112.443136e6, ("recon", 4): 243.891968e6 + 49.104128e6,
+    ("limiter", 8): 293.396224e6 + 305.403392e6, ("limiter", 4): 168.634880e6 + 129.079040e6,
+    ("corr_flux", 8): 495.858688e6 + 207.361024e6, ("corr_flux", 4): 328.393984e6 + 95.449600e6,
+    ("corr_cell", 8): 468.417024e6 + 68.509184e6, ("corr_cell", 4): 292.142336e6 + 51.723520e6,
+    ("pred_flux", 8): 181.941760e6 + 188.923392e6, ("pred_flux", 4): 170.661376e6 + 86.100992e6,
+    ("pred_cell", 8): 343.107840e6 + 35.037440e6, ("pred_cell", 4): 195.695360e6 + 17.731584e6,
+    ("recon", 8): 259.623680e6 + 111.263232e6, ("recon", 4): 256.654848e6 + 47.741184e6,
 }
 # FP64 floating-point operations per launch on the same 64^3 launches (ncu
 # thread-instruction counts: 2 per DFMA, 1 per DADD and DMUL; this includes

@@ -1351,8 +1351,8 @@ FVM_CELL_LOOP_(FVM_GATHER_UNR)
 // 12^3 to 20^3 take the same time either way (75.3 and 75.7 us, 87.5 and
 // 87.5), 32^3 gain 1%, hence SUM_CELLS.  Loops unrolled by 1, 3 or 4 and
 // blocks of 112 or 448 threads measured slower (992, 907, 926, 899, 923 us
-// against 880).  FP32 keeps one thread per cell: its records are half as
-// long, and the compensated sums' state has to travel with them.
+// against 880).  FP32 keeps one thread per cell; the form has not been
+// measured there.
 template <bool SKIPJ>
 __global__ void __launch_bounds__(SUM_BLOCK) k_cell_sums(int n, const int *FVM_RESTRICT off,
     const int2 *FVM_RESTRICT lfj, const double *FVM_RESTRICT fcon, const unsigned char *FVM_RESTRICT fcode,

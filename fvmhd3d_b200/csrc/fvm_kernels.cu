@@ -212,8 +212,10 @@ struct fvm_ctx {
   LearnBuf lb{};
   float h_norm[48];  // standardisation of the network's inputs and outputs (fvm_mlp_set_norm)
   // launch choices of the autotuner (fvm_autotune); the defaults are the
-  // tuned values of the 16^3 to 128^3 blasts (against 64, 64, 64: FP64 steps 1
-  // to 3% shorter, FP32 the same)
+  // tuned values of global steps of the 16^3 to 128^3 blasts (against 64, 64,
+  // 64: FP64 steps 1 to 3% shorter, FP32 the same); in partial steps of 16^3 to
+  // 80^3 blasts 32, 64 and 128 threads in the face and cell kernels are within
+  // 2% of each other, either way
   struct {
     int lim_staged = FVM_LIMITER_STAGE;  // staged limiter (shared-memory face records) or one record per thread
     int bs_face = 32;    // threads per block of the face kernels

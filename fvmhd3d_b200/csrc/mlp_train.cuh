@@ -131,7 +131,7 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const float *v) {
 // the last 128 columns.  Training amplifies round-off (after 40 steps 1e-7 is
 // 1e-4), so the order of every sum is fixed: by the 16 rows of a product
 // within a CTA's rows, by CTA, and for the bias gradients by row.
-// A step of 8,192 rows takes 42 us here and 44 in k_update; as separate
+// A step of 8,192 rows takes 43 us here and 44 in k_update; as separate
 // products, elementwise passes and column sums it was 32 launches and 1.25 ms.
 // err bit 4: an mbarrier wait gave up.
 static __global__ void __launch_bounds__(THREADS, 1) k_fwd_bwd(int rows, int per, long long n, const float *__restrict__ X,

@@ -336,7 +336,9 @@ int fvm_autotune(fvm_ctx *c, int shared, int steps, int *choice);
  * limiter to the reconstruction as one cooperative launch with grid-wide
  * barriers between the stages; larger steps take the stage kernels.  The
  * choice is made on the device each step; both give the same results.
- * 0 (the default) turns it off.  Learned-flux mode and per-kernel profiling
+ * 0 (the default) turns it off: the stage kernels have come to take as long or
+ * less on all but the smallest steps (100K-cell disk: 30 cells 131 and 136 us
+ * in FP64, 142 and 136 in FP32; 11,000 cells 240 and 269).  Learned-flux mode and per-kernel profiling
  * always take the stage kernels.  Has no counterpart in the reference (a
  * GPU batching of its per-rung fluid_update sequence). */
 int fvm_set_fused(fvm_ctx *c, int max_cells);
