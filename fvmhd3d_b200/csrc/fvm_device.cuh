@@ -1808,9 +1808,9 @@ __device__ __forceinline__ void timestep_group(Params P, const int *FVM_RESTRICT
   if ((threadIdx.x & 31) == 0 && vmin < FVM_HUGE) atomic_min_pos(dmin, vmin);
 }
 
-// Also starts the step's adjust_timesteps over from nothing: its counters and
-// flags, and (partial steps: work not null) its marks and work lists, cleared
-// for the involved cells only: every mark, work list and replay write of the
+// Also starts adjust_timesteps over from nothing in the steps that run it (work
+// not null): its counters and flags, and its marks and work lists, cleared for
+// the involved cells only: every mark, work list and replay write of the
 // step lands on one of them, and every reader walks them only.
 __global__ void k_timestep(int n, Params P, const int *FVM_RESTRICT off, const int2 *FVM_RESTRICT lfj,
                            const unsigned char *FVM_RESTRICT act,
@@ -1825,10 +1825,10 @@ __global__ void k_timestep(int n, Params P, const int *FVM_RESTRICT off, const i
   // repeats the cell's own terms, and on a full step that costs more than the
   // shorter face walk gains (0.26 -> 0.69 ms on the 128^3 blast)
   const int gt = blockIdx.x * blockDim.x + threadIdx.x, gn = gridDim.x * blockDim.x;
-  if (gt < 4) S->iscal[4 + gt] = 0;
-  if (gt < 8) aflag[gt] = 0;
   const int ninv = clist ? S->ninv : 0;
-  if (work) {
+  if (work) {  // (a global step leaves the last individual one's counters to be asked for)
+    if (gt < 4) S->iscal[4 + gt] = 0;
+    if (gt < 8) aflag[gt] = 0;
     const bool lst = ninv != n;  // every cell involved: the list is the identity
     for (int t = gt; t < ninv; t += gn) {
       const int i = lst ? clist[t] : t;
